@@ -18,8 +18,8 @@
 // Forward kernels either write per-pixel losses, or only the [sum, count] record
 // (deterministic last-block reduction), or both.  Backward kernels recompute the softmax
 // and scale by the upstream gradient and the (device-resident) valid count.
-#include "softmax_core.cuh"
 #include "pipeline.cuh"
+#include "softmax_params.cuh"
 
 #include <stdlib.h>
 
@@ -31,31 +31,6 @@ constexpr size_t kTileTargetBytes = 48 * 1024;
 constexpr size_t kSmemLimit = 200 * 1024;
 
 constexpr int kPcMaxC = 256;     // classes the kPC fused step holds weights for
-
-struct SoftmaxParams {
-    const void *logits;
-    const int64_t *labels;
-    void *losses;            // [N, M] dtype or null
-    void *grads;             // [N, C, M] dtype (backward)
-    const void *grad_out;    // see grad_mode
-    int grad_mode;
-    const double *denom;
-    void *workspace;
-    ReduceRecord *out;
-    float4 *stats;           // [N*M] per-pixel statistics: written by the chunked forward, read by
-                             // the chunked backward (null: not wanted / not available)
-    int64_t N, C, M;
-    int64_t ignore;
-    LossConsts k;
-    // tile geometry
-    int TP, KS, CB, nbox, rows;
-    int nbx;                 // boxes of TP pixels per tile (pair kernel)
-    int stages;              // ring depth of the pipelined kernels
-    int64_t tiles_per_image, total_tiles;
-    int defer;               // cross-GPU sum of the fused step: post only (see grid_reduce_finish)
-    int after_count;         // fused step launched as a programmatic dependent of the label count
-    const float *chan_w;     // kPC: class weights [C] (device)
-};
 
 // ------------------------------------------------------------------ tile regime
 
@@ -1561,7 +1536,6 @@ rows_pipe_kernel(const SoftmaxParams prm) {
 
 // -------------------------------------------------------------------- dispatch
 
-inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // ------------------------------------------------- rows regime, forward: one warp per row
 //
@@ -1750,338 +1724,6 @@ rows_warp_fwd_kernel(const SoftmaxParams prm) {
     if (REDUCE) grid_reduce_finish(acc_loss, acc_cnt, prm.workspace, prm.out, sh_red, kTagSum, prm.defer != 0);
 }
 
-// ------------------------------------------------------------- short-rows regime
-// M == 1 with up to 2048 channels: [N, C] classification inputs and channels-last images, where
-// every pixel is a row of C contiguous logits (C x element size need not be a multiple of 16).  A
-// stage holds R = 256 / TPR consecutive rows -- ONE contiguous run of R * C elements, moved by one bulk copy in and, in
-// backward, one bulk copy out (R is a multiple of 8 and an element has 2 or 4 bytes, so every run starts and ends on 16 bytes) --
-// together with the R labels.  TPR adjacent lanes (1 to 32: at most 32 channels per lane up to
-// 1024 channels, 64 beyond) share a row and combine their statistics with shuffles: no block barrier, no shared-memory
-// exchange.  The last rows of the input (fewer than R) have no 16-byte guarantee: the
-// compute threads move them with plain loads and stores.
-constexpr int kShortCompute = 256;
-constexpr int kShortBlock = kShortCompute + 64;
-constexpr int kShortRowsMaxC = 2048;          // a warp per row, 64 channels per lane
-
-// Statistics of a row combined over its TPR adjacent lanes.  `mask` names exactly those lanes: the
-// lanes of a row take the same branches (a row is valid or ignored as a whole), other rows of
-// the warp may be elsewhere.
-template <int KIND> struct LaneMerge;
-template <> struct LaneMerge<kLSR> {
-    static __device__ __forceinline__ void s1(Stat1<kLSR> &a, int tpr, unsigned mask) {
-        for (int o = tpr >> 1; o > 0; o >>= 1) a.m = fmaxf(a.m, __shfl_xor_sync(mask, a.m, o));
-    }
-    static __device__ __forceinline__ void s2(Stat2<kLSR> &b, int tpr, unsigned mask) {
-        for (int o = tpr >> 1; o > 0; o >>= 1) {
-            b.s += __shfl_xor_sync(mask, b.s, o);
-            b.sx += __shfl_xor_sync(mask, b.sx, o);
-            b.xl += __shfl_xor_sync(mask, b.xl, o);
-        }
-    }
-};
-template <> struct LaneMerge<kLMargin> {
-    static __device__ __forceinline__ void s1(Stat1<kLMargin> &a, int tpr, unsigned mask) {
-        for (int o = tpr >> 1; o > 0; o >>= 1) {
-            a.m_no = fmaxf(a.m_no, __shfl_xor_sync(mask, a.m_no, o));
-            a.xl = fmaxf(a.xl, __shfl_xor_sync(mask, a.xl, o));
-        }
-    }
-    static __device__ __forceinline__ void s2(Stat2<kLMargin> &b, int tpr, unsigned mask) {
-        for (int o = tpr >> 1; o > 0; o >>= 1) {
-            b.s_no += __shfl_xor_sync(mask, b.s_no, o);
-            b.sde += __shfl_xor_sync(mask, b.sde, o);
-            b.sd += __shfl_xor_sync(mask, b.sd, o);
-        }
-    }
-};
-
-template <typename T, int KIND, bool BWD, bool REDUCE>
-__global__ void __launch_bounds__(kShortBlock)
-rows_multi_kernel(const SoftmaxParams prm) {
-    extern __shared__ unsigned char smem_raw[];
-    __shared__ PipeBarriers bars;
-    __shared__ double sh_red[64];
-
-    const int C = static_cast<int>(prm.C), NS = prm.stages, TPR = prm.KS;
-    const int R = kShortCompute / TPR;                       // rows per stage
-    unsigned char *base = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
-    const size_t label_off = (size_t(R) * C * sizeof(T) + 127) & ~size_t(127);
-    const size_t stage_bytes = label_off + size_t(R) * sizeof(int64_t);
-    const int tid = threadIdx.x;
-    unsigned *status = prm.workspace ? reinterpret_cast<unsigned *>(prm.workspace) + 1 : nullptr;
-    const int64_t n_stages = (prm.N + R - 1) / R;
-    const uint32_t full_bytes = uint32_t(R) * C * sizeof(T);
-
-    pipe_init<kShortCompute, BWD>(bars, NS);
-    const int64_t first = blockIdx.x, stride = gridDim.x;
-    double acc_loss = 0.0, acc_cnt = 0.0;
-
-    if (tid == kShortCompute) {
-        int k = 0;
-        for (int64_t st = first; st < n_stages; st += stride, ++k) {
-            const int s = k % NS;
-            if (k >= NS && !mbar_wait_bounded(&bars.empty[s], ((k / NS) - 1) & 1, status)) break;
-            const int64_t row0 = st * R;
-            if (prm.N - row0 >= R) {
-                unsigned char *stage = base + s * stage_bytes;
-                const unsigned char *src = static_cast<const unsigned char *>(prm.logits) + row0 * C * sizeof(T);
-                mbar_expect_tx(&bars.full[s], full_bytes + uint32_t(R) * sizeof(int64_t));
-                for (uint32_t off = 0; off < full_bytes; off += 32768u) {
-                    const uint32_t nb = full_bytes - off < 32768u ? full_bytes - off : 32768u;
-                    bulk_load_1d(stage + off, src + off, nb, &bars.full[s]);
-                }
-                bulk_load_1d(stage + label_off, prm.labels + row0, uint32_t(R) * sizeof(int64_t), &bars.full[s]);
-            } else {
-                mbar_expect_tx(&bars.full[s], 0);            // ragged end: the compute threads fetch it themselves
-            }
-        }
-    } else if (BWD && tid == kShortCompute + 32) {
-        int k = 0;
-        for (int64_t st = first; st < n_stages; st += stride, ++k) {
-            const int s = k % NS;
-            if (!mbar_wait_bounded(&bars.ready[s], (k / NS) & 1, status)) break;
-            const int64_t row0 = st * R;
-            if (prm.N - row0 >= R) {
-                const unsigned char *stage = base + s * stage_bytes;
-                unsigned char *dst = static_cast<unsigned char *>(prm.grads) + row0 * C * sizeof(T);
-                for (uint32_t off = 0; off < full_bytes; off += 32768u) {
-                    const uint32_t nb = full_bytes - off < 32768u ? full_bytes - off : 32768u;
-                    bulk_store_1d(dst + off, stage + off, nb);
-                }
-                bulk_commit();
-                bulk_wait_read_all();
-            }
-            mbar_arrive(&bars.empty[s]);
-        }
-        bulk_wait_all();
-    } else if (tid < kShortCompute) {
-        const int lane = tid & 31;
-        const int rowl = tid / TPR, t = tid % TPR;           // my row inside a stage, my lane inside the row
-        // A lane visits the units (channels, or channel pairs) u = c * TPR + t of its row, chunk c
-        // after chunk c.  Few lanes per row and an even C: the rows of a warp lie an even number of
-        // words apart and would share banks, so the walk starts at a chunk that depends on the row
-        // and wraps around (same trip count in every lane: no divergence).  Otherwise (odd C, or
-        // 8+ lanes per row = few rows per warp) a plain strided loop.
-        const bool rotate = TPR <= 4 && (C & 1) == 0;
-        const int chunks_c = (C + TPR - 1) / TPR, chunks_p = ((C >> 1) + TPR - 1) / TPR;
-        const int rot_c = rotate ? rowl % chunks_c : 0, rot_p = (rotate && chunks_p > 0) ? rowl % chunks_p : 0;
-        auto walk_units = [&](int n, int chunks, int rot, auto &&body) {
-            if (!rotate && TPR == 1) {
-#pragma unroll 4
-                for (int u = 0; u < n; ++u) body(u);            // (unit stride: immediate offsets after unrolling)
-            } else if (!rotate) {
-#pragma unroll 4
-                for (int u = t; u < n; u += TPR) body(u);
-            } else {
-                int c = rot;
-#pragma unroll 4
-                for (int i = 0; i < chunks; ++i) {
-                    const int u = c * TPR + t;
-                    if (u < n) body(u);
-                    c = (c + 1 == chunks) ? 0 : c + 1;
-                }
-            }
-        };
-        auto walk = [&](auto &&body) { walk_units(C, chunks_c, rot_c, body); };
-        const unsigned row_mask = (TPR == 32 ? 0xffffffffu : ((1u << TPR) - 1u)) << (lane & ~(TPR - 1));
-        const T *gout = static_cast<const T *>(prm.grad_out);
-        T *losses = static_cast<T *>(prm.losses);
-        const LossConsts kc = prm.k;
-        float gscale = 1.f;
-        if (BWD && REDUCE) pdl_wait();                       // (see tile_pair_kernel)
-        if (BWD) gscale = uniform_grad_scale(prm.grad_out, prm.grad_mode, prm.denom);
-        int k = 0;
-        for (int64_t st = first; st < n_stages; st += stride, ++k) {
-            const int s = k % NS;
-            bool ok = true;
-            if (lane == 0) ok = mbar_wait_bounded(&bars.full[s], (k / NS) & 1, status);
-            // (the ragged last stage needs all compute threads at a named barrier, which has no
-            // time limit: every stage's decision to go on is taken by all of them together)
-            if (!compute_all(ok, kShortCompute)) break;
-            const int64_t row0 = st * R;
-            const int nrows = prm.N - row0 >= R ? R : int(prm.N - row0);
-            const bool ragged = nrows < R;
-            T *tile = reinterpret_cast<T *>(base + s * stage_bytes);
-            int64_t *tile_labels = reinterpret_cast<int64_t *>(base + s * stage_bytes + label_off);
-            if (ragged) {
-                const T *src = static_cast<const T *>(prm.logits) + row0 * C;
-                for (int e = tid; e < nrows * C; e += kShortCompute) tile[e] = src[e];
-                for (int e = tid; e < nrows; e += kShortCompute) tile_labels[e] = prm.labels[row0 + e];
-                compute_sync(kShortCompute);
-            }
-            const bool live = rowl < nrows;
-            const int64_t row = row0 + rowl;
-            const int64_t lb = live ? tile_labels[rowl] : prm.ignore;
-            const bool valid = live && lb != prm.ignore;
-            const int lbi = valid ? ((lb >= 0 && lb < C) ? int(lb) : -2) : -1;
-            T *rp = tile + size_t(rowl) * C;
-            if (KIND == kLSR && valid && (C & 1) == 0) {
-                // Label smooth, even C: the lane's channels as adjacent PAIRS (one 8-byte -- half
-                // types 4-byte -- access and packed fp32x2 arithmetic per pair), e^{x-m} kept in the
-                // tile between the sum and the gradient (one exponential per element), the target
-                // term added by the lane that owns the label's pair (tile_pair_kernel's scheme).
-                const int npair = C >> 1;
-                const float xl = lbi >= 0 ? to_f32(rp[lbi]) : 0.f;
-                __syncwarp(row_mask);                          // all of the row's lanes hold x_lb before e^{x-m} overwrites it
-                float2 m2 = splat2(kNegInf);
-                walk_units(npair, chunks_p, rot_p, [&](int q) { m2 = max2(m2, ld_pair(rp + 2 * q)); });
-                float m = fmaxf(m2.x, m2.y);
-                for (int o = TPR >> 1; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(row_mask, m, o));
-                pk_t psum = psplat(0.f), psx = psplat(0.f);
-                {
-                    const pk_t nml = psplat(-m * kLog2e), l2e = psplat(kLog2e);
-                    walk_units(npair, chunks_p, rot_p, [&](int q) {
-                        const pk_t x = ld_pk(rp + 2 * q);
-                        const pk_t e = pex2(pfma(x, l2e, nml));
-                        psum = padd(psum, e);
-                        psx = padd(psx, x);
-                        if (BWD) st_pk(rp + 2 * q, e);
-                    });
-                }
-                float2 s2v = upk2(psum), sxv = upk2(psx);
-                float sum = s2v.x + s2v.y, sx = sxv.x + sxv.y;
-                for (int o = TPR >> 1; o > 0; o >>= 1) {
-                    sum += __shfl_xor_sync(row_mask, sum, o);
-                    sx += __shfl_xor_sync(row_mask, sx, o);
-                }
-                const float loss = kc.sumy * (m + __logf(sum)) - kc.lb_neg * sx - (kc.lb_pos - kc.lb_neg) * xl;
-                if (t == 0) {
-                    if (!BWD && losses) losses[row] = from_f32<T>(loss);
-                    if (REDUCE) {
-                        acc_loss += double(loss);
-                        acc_cnt += 1.0;
-                    }
-                }
-                if (BWD) {
-                    float psc = gscale;
-                    if (prm.grad_mode == 2) psc *= to_f32(gout[row]);
-                    // g = (sumy e / s - lb_neg) scale, then the target's lb_neg -> lb_pos
-                    const pk_t pa = psplat(kc.sumy * __fdividef(psc, sum)), pb = psplat(-kc.lb_neg * psc);
-                    walk_units(npair, chunks_p, rot_p, [&](int q) { st_pk(rp + 2 * q, pfma(ld_pk(rp + 2 * q), pa, pb)); });
-                    if (lbi >= 0 && (lbi >> 1) % TPR == t)
-                        rp[lbi] = from_f32<T>(to_f32(rp[lbi]) - (kc.lb_pos - kc.lb_neg) * psc);
-                }
-            } else if (KIND == kLMargin && valid && lbi >= 0 && (C & 1) == 0) {
-                // Large margin, even C: channel pairs and packed arithmetic as above, the target
-                // handled as in tile_pair_kernel: its logit is parked at -FLT_MAX for the maximum
-                // sweep and at min(x_lb, m') for the sum sweep, its terms are then taken back out of
-                // the sums (s' >= 1 >= e^{min(x_lb - m', 0)}: nothing cancels), and its gradient
-                // overwrites what the sweep left there.
-                const int npair = C >> 1;
-                const float xl = to_f32(rp[lbi]);
-                __syncwarp(row_mask);                          // all of the row's lanes hold x_lb before it is parked
-                const bool owner = (lbi >> 1) % TPR == t;      // my walk visits the label's pair
-                if (owner) rp[lbi] = from_f32<T>(sizeof(T) == 2 ? -65504.f : kNegInf);
-                float2 m2 = splat2(kNegInf);
-                walk_units(npair, chunks_p, rot_p, [&](int q) { m2 = max2(m2, ld_pair(rp + 2 * q)); });
-                float m = fmaxf(m2.x, m2.y);
-                for (int o = TPR >> 1; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(row_mask, m, o));
-                const float cl = fminf(xl, m);
-                if (owner) rp[lbi] = from_f32<T>(cl);
-                const pk_t pnegm = psplat(-m), l2e = psplat(kLog2e);
-                pk_t psum = psplat(0.f), psde = psplat(0.f), psx = psplat(0.f);
-                walk_units(npair, chunks_p, rot_p, [&](int q) {
-                    const pk_t x = ld_pk(rp + 2 * q);
-                    const pk_t d = padd(x, pnegm);
-                    const pk_t e = pex2(pmul(d, l2e));
-                    psum = padd(psum, e);
-                    psde = pfma(d, e, psde);
-                    psx = padd(psx, x);
-                });
-                const float2 v1 = upk2(psum), v2 = upk2(psde), v3 = upk2(psx);
-                float sum = v1.x + v1.y, sde = v2.x + v2.y, sx = v3.x + v3.y;
-                for (int o = TPR >> 1; o > 0; o >>= 1) {
-                    sum += __shfl_xor_sync(row_mask, sum, o);
-                    sde += __shfl_xor_sync(row_mask, sde, o);
-                    sx += __shfl_xor_sync(row_mask, sx, o);
-                }
-                // (half tiles hold the parked value rounded to T: use what the sweep read)
-                const float clr = to_f32(from_f32<T>(cl));
-                const float dc = clr - m;
-                const float ec = ex2f(dc * kLog2e);
-                const float s_no = sum - ec;
-                const float sde_no = sde - dc * ec;
-                const float sd = (sx - clr) - float(C - 1) * m;
-                const float inv_s = __fdividef(1.f, s_no);
-                const float sqx = sde_no * inv_s;
-                const float mm = fmaxf(m, xl);
-                const float e_no = s_no * ex2f((m - mm) * kLog2e);
-                const float e_lb = ex2f((xl - mm) * kLog2e);
-                const float s_all = e_no + e_lb;
-                const float rr = __fdividef(e_no, s_all);
-                const float loss = (mm + __logf(s_all)) - xl + kc.half_lam * (sqx - kc.a * sd);
-                if (t == 0) {
-                    if (!BWD && losses) losses[row] = from_f32<T>(loss);
-                    if (REDUCE) {
-                        acc_loss += double(loss);
-                        acc_cnt += 1.0;
-                    }
-                }
-                if (BWD) {
-                    float psc = gscale;
-                    if (prm.grad_mode == 2) psc *= to_f32(gout[row]);
-                    // g_j = scale (r q + lam/2 (q (d + 1 - sqx) - a)) = q (A + B d) + Cc,  q = e^d / s'
-                    const pk_t pqa = psplat((rr + kc.half_lam * (1.f - sqx)) * psc), pqb = psplat(kc.half_lam * psc);
-                    const pk_t pcc = psplat(-kc.half_lam * kc.a * psc), pqs = psplat(inv_s);
-                    walk_units(npair, chunks_p, rot_p, [&](int q) {
-                        const pk_t d = padd(ld_pk(rp + 2 * q), pnegm);
-                        const pk_t qq = pmul(pex2(pmul(d, l2e)), pqs);
-                        st_pk(rp + 2 * q, pfma(qq, pfma(pqb, d, pqa), pcc));
-                    });
-                    if (owner) rp[lbi] = from_f32<T>(-rr * psc);
-                }
-            } else if (valid) {
-                Stat1<KIND> s1;
-                s1.init();
-                walk([&](int j) { s1.add(to_f32(rp[j]), j == lbi); });
-                LaneMerge<KIND>::s1(s1, TPR, row_mask);
-                Stat2<KIND> s2;
-                s2.init();
-                walk([&](int j) { s2.add(to_f32(rp[j]), j == lbi, s1); });
-                LaneMerge<KIND>::s2(s2, TPR, row_mask);
-                PixelFinal<KIND> fin;
-                fin.finish(s1, s2, kc);
-                if (t == 0) {
-                    if (!BWD && losses) losses[row] = from_f32<T>(fin.loss);
-                    if (REDUCE) {
-                        acc_loss += double(fin.loss);
-                        acc_cnt += 1.0;
-                    }
-                }
-                if (BWD) {
-                    float psc = gscale;
-                    if (prm.grad_mode == 2) psc *= to_f32(gout[row]);
-                    walk([&](int j) { rp[j] = from_f32<T>(fin.grad(to_f32(rp[j]), j == lbi, kc) * psc); });
-                }
-            } else if (live) {
-                if (!BWD && losses && t == 0) losses[row] = from_f32<T>(0.f);
-                if (BWD)
-                    for (int p = t; p < C; p += TPR) rp[p] = from_f32<T>(0.f);
-            }
-            if (!BWD) {
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&bars.empty[s]);
-            } else {
-                if (ragged) {
-                    compute_sync(kShortCompute);
-                    T *dst = static_cast<T *>(prm.grads) + row0 * C;
-                    for (int e = tid; e < nrows * C; e += kShortCompute) dst[e] = tile[e];
-                } else {
-                    fence_proxy_async_smem();
-                }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&bars.ready[s]);
-            }
-        }
-    }
-    if (REDUCE) grid_reduce_finish(acc_loss, acc_cnt, prm.workspace, prm.out, sh_red, kTagSum, prm.defer != 0);
-}
-
-// The layouts rows_multi_kernel takes.
-inline bool short_rows_eligible(const void *logits, const void *io, const void *labels, int64_t N, int64_t C, int64_t M) {
-    return M == 1 && N >= 1 && C >= 1 && C <= kShortRowsMaxC && aligned16(logits) && aligned16(io) && aligned16(labels);
-}
-
 // ------------------------------------------------------------- any-alignment spatial regime
 // M > 1 where the rows of a channel do not start on 16 bytes (M not a multiple of 4 floats: 769 x
 // 769 or 713 x 713 crops) or the pointers are not aligned: no tensor map, no bulk copy.  The 256
@@ -2221,17 +1863,6 @@ int launch_spatial_any(const SoftmaxParams &prm, cudaStream_t stream) {
     else if (prm.C <= 160) launch_kernel(spatial_any_kernel<KIND, BWD, REDUCE, 4, 40>, gd, bd, 0, stream, dep, prm);
     else launch_kernel(spatial_any_kernel<KIND, BWD, REDUCE, 8, 40>, gd, bd, 0, stream, dep, prm);
     return launch_status("softmax any-alignment kernel launch");
-}
-
-// Integer tuning override from the environment (tile size, ring depth, blocks per SM);
-// unset or unparsable -> the default.
-
-template <typename K> int set_smem(K kernel, size_t bytes) {
-    if (bytes > 40 * 1024) {   // static shared memory shares the default 48 KiB
-        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)) != cudaSuccess)
-            return launch_status("cudaFuncSetAttribute(max dynamic shared memory)");
-    }
-    return B200_OK;
 }
 
 // True when the chunked kernels (tile_chunk_fwd_kernel / tile_chunk_bwd_kernel) take the call:
@@ -2399,31 +2030,8 @@ int launch_regime(SoftmaxParams prm, int dtype, cudaStream_t stream) {
         set_error("pc softmax step: this layout has no fused step");
         return B200_ERR_UNSUPPORTED;
     } else {
-    if (short_rows_eligible(prm.logits, io, prm.labels, prm.N, prm.C, prm.M)) {
-        // ---- short-rows regime
-        // at most 32 channels per lane, 3 stages in backward (measured on the fused steps of configs 1
-        // and 3 in channels-last: 0.148 / 0.797 ms; 2 or 4 stages 0.162 / 0.93-0.95 ms; 16 channels per
-        // lane doubles config 1's time; 40 per lane and 2 stages: 0.163 / 0.760 ms)
-        int tpr = 1;
-        while (tpr < 32 && (prm.C + tpr - 1) / tpr > 32) tpr <<= 1;
-        prm.KS = tpr;
-        const int R = kShortCompute / tpr;
-        const size_t label_off = (size_t(R) * prm.C * es + 127) & ~size_t(127);
-        const size_t stage_bytes = label_off + size_t(R) * sizeof(int64_t);
-        prm.stages = (BWD && stage_bytes <= size_t(36) * 1024) ? 3 : 2;
-        const size_t smem = 128 + size_t(prm.stages) * stage_bytes;
-        int per_sm = int((224 * 1024) / (smem + 2048));
-        if (per_sm > 4) per_sm = 4;
-        if (per_sm < 1) per_sm = 1;
-        const int64_t n_stages = (prm.N + R - 1) / R;
-        int64_t grid = int64_t(sms) * per_sm;
-        if (grid > n_stages) grid = n_stages;
-        if (grid > kMaxPartials) grid = kMaxPartials;
-        auto kern = rows_multi_kernel<T, KIND, BWD, REDUCE>;
-        int rc;
-        if ((rc = set_smem(kern, smem)) != B200_OK) return rc;
-        launch_kernel(kern, dim3(unsigned(grid)), dim3(kShortBlock), smem, stream, BWD && REDUCE && prm.after_count, prm);
-        return launch_status("softmax short-rows kernel launch");
+    if (short_rows_eligible(es, prm.logits, io, prm.labels, prm.N, prm.C, prm.M)) {
+        return launch_short_rows(KIND, BWD, dtype, prm, stream);
     }
     if constexpr (!BWD) {
         // ---- rows regime, forward, long rows: one warp per row, streamed (any row length)
@@ -2618,7 +2226,7 @@ inline bool fused_step_eligible(size_t es, const void *logits, const void *grads
                                 int64_t C, int64_t M) {
     if (N < 1 || M < 1) return false;
     if (M == 1) {
-        if (C <= kShortRowsMaxC && aligned16(logits) && aligned16(grads) && aligned16(labels)) return true;   // short rows
+        if (short_rows_eligible(es, logits, grads, labels, N, C, M)) return true;
         return size_t(C) * es + 1024 <= kSmemLimit && (size_t(C) * es) % 16 == 0 && aligned16(logits) && aligned16(grads);
     }
     if (size_t(C) * 32 * es + 8192 > kSmemLimit) return false;
@@ -2706,110 +2314,6 @@ lsr_resident_step_kernel(const SoftmaxParams prm) {
     grid_reduce_finish(double(acc), double(cnt), prm.workspace, prm.out, sh_red, kTagSum, prm.defer != 0);
 }
 
-// Label-smooth training step over classification rows (M == 1, float32, C a multiple of 4 between
-// 64 and 2048, 16-byte aligned pointers): a warp owns a row and keeps it in registers -- NV 16-byte
-// vectors per lane, all of a lane's loads in flight together -- so the logits are read once and the
-// gradient is written once, with no shared memory and no barrier before the final reduction.  The
-// target's logit is fetched again (one 4-byte load per row) and its gradient is a 4-byte store by
-// the lane that wrote the vector around it.
-template <int NV>
-__global__ void __launch_bounds__(kResidentThreads, NV <= 8 ? 3 : 2)
-lsr_rows_resident_step_kernel(const SoftmaxParams prm) {
-    __shared__ double sh_red[64];
-    const float4 *x = static_cast<const float4 *>(prm.logits);
-    float4 *grads = static_cast<float4 *>(prm.grads);
-    const int lane = threadIdx.x & 31;
-    const int C = prm.k.C, nvec = C >> 2;
-    const int64_t warps = int64_t(gridDim.x) * (kResidentThreads / 32);
-    pdl_wait();                                    // the divisor comes from the label count in front
-    const float gs = uniform_grad_scale(nullptr, 0, prm.denom);
-    const float dpn = prm.k.lb_pos - prm.k.lb_neg;
-    float acc = 0.f, cnt = 0.f;
-    for (int64_t r = int64_t(blockIdx.x) * (kResidentThreads / 32) + (threadIdx.x >> 5); r < prm.N; r += warps) {
-        const float4 *xr = x + r * nvec;
-        float4 xv[NV];
-#pragma unroll
-        for (int i = 0; i < NV; ++i) {
-            const int v = lane + 32 * i;
-            if (v < nvec) xv[i] = __ldcs(xr + v);
-        }
-        const int64_t lb = __ldg(prm.labels + r);
-        const bool valid = lb != prm.ignore;
-        // (a label outside [0, C) that is not the ignore value is undefined in the reference: no target term here)
-        const int lbi = (valid && lb >= 0 && lb < C) ? int(lb) : -1;
-        const float xl = lbi >= 0 ? __ldg(static_cast<const float *>(prm.logits) + r * C + lbi) : 0.f;
-        float4 *grow = grads + r * nvec;
-        if (!valid) {                              // (uniform over the warp)
-#pragma unroll
-            for (int i = 0; i < NV; ++i) {
-                const int v = lane + 32 * i;
-                if (v < nvec) __stcs(grow + v, make_float4(0.f, 0.f, 0.f, 0.f));
-            }
-            continue;
-        }
-        float m = kNegInf, sx = 0.f;
-#pragma unroll
-        for (int i = 0; i < NV; ++i) {
-            if (lane + 32 * i < nvec) {
-                m = fmaxf(fmaxf(m, fmaxf(xv[i].x, xv[i].y)), fmaxf(xv[i].z, xv[i].w));
-                sx += (xv[i].x + xv[i].y) + (xv[i].z + xv[i].w);
-            }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-        const float nm2 = -m * kLog2e;
-        float s = 0.f;
-#pragma unroll
-        for (int i = 0; i < NV; ++i) {
-            if (lane + 32 * i < nvec) {
-                xv[i].x = ex2f(fmaf(xv[i].x, kLog2e, nm2));         // e^{x-m} takes x's place
-                xv[i].y = ex2f(fmaf(xv[i].y, kLog2e, nm2));
-                xv[i].z = ex2f(fmaf(xv[i].z, kLog2e, nm2));
-                xv[i].w = ex2f(fmaf(xv[i].w, kLog2e, nm2));
-                s += (xv[i].x + xv[i].y) + (xv[i].z + xv[i].w);
-            }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            s += __shfl_xor_sync(0xffffffffu, s, o);
-            sx += __shfl_xor_sync(0xffffffffu, sx, o);
-        }
-        if (lane == 0) {
-            acc += prm.k.sumy * (m + __log2f(s) * kLn2) - prm.k.lb_neg * sx - dpn * xl;
-            cnt += 1.f;
-        }
-        const float a = prm.k.sumy * __fdividef(gs, s), b = -prm.k.lb_neg * gs;
-#pragma unroll
-        for (int i = 0; i < NV; ++i) {
-            const int v = lane + 32 * i;
-            if (v < nvec)
-                __stcs(grow + v, make_float4(fmaf(xv[i].x, a, b), fmaf(xv[i].y, a, b), fmaf(xv[i].z, a, b), fmaf(xv[i].w, a, b)));
-        }
-        // target: (sumy e_l / s - lb_pos) gs, by the lane whose vector store covers it (program order)
-        if (lbi >= 0 && ((lbi >> 2) & 31) == lane)
-            reinterpret_cast<float *>(grow)[lbi] = fmaf(ex2f(fmaf(xl, kLog2e, nm2)), a, -prm.k.lb_pos * gs);
-    }
-    grid_reduce_finish(double(acc), double(cnt), prm.workspace, prm.out, sh_red, kTagSum, prm.defer != 0);
-}
-
-inline bool rows_resident_step_eligible(int kind, int dtype, const void *logits, const void *grads, const void *labels,
-                                        int64_t N, int64_t C, int64_t M) {
-    return kind == kLSR && dtype == B200_F32 && M == 1 && N >= 1 && C % 4 == 0 && C >= 64 && C <= 2048 &&
-           aligned16(logits) && aligned16(grads) && labels != nullptr;
-}
-
-int launch_rows_resident_step(const SoftmaxParams &prm, cudaStream_t stream) {
-    int64_t grid = (prm.N + kResidentThreads / 32 - 1) / (kResidentThreads / 32);
-    const int64_t cap = int64_t(sm_count()) * (prm.C <= 1024 ? 3 : 2);   // all blocks resident: one reduction barrier per block
-    if (grid > cap) grid = cap;
-    const dim3 gd{unsigned(grid)}, bd(kResidentThreads);
-    const bool dep = prm.after_count != 0;
-    if (prm.C <= 256) launch_kernel(lsr_rows_resident_step_kernel<2>, gd, bd, 0, stream, dep, prm);
-    else if (prm.C <= 1024) launch_kernel(lsr_rows_resident_step_kernel<8>, gd, bd, 0, stream, dep, prm);
-    else launch_kernel(lsr_rows_resident_step_kernel<16>, gd, bd, 0, stream, dep, prm);
-    return launch_status("label-smooth resident rows step launch");
-}
-
 inline bool aligned8(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 7u) == 0; }
 
 // The layouts lsr_resident_step_kernel takes, and the sizes it wins at: up to ~40 M elements its
@@ -2879,8 +2383,6 @@ int fused_step(const char *who, const void *logits, const int64_t *labels, void 
     prm.defer = defer & B200_STEP_DEFER;
     prm.after_count = (denom != nullptr && (defer & B200_STEP_AFTER_COUNT)) ? 1 : 0;
     if (resident) return launch_resident_step(prm, static_cast<cudaStream_t>(stream));
-    if (rows_resident_step_eligible(KIND, dtype, logits, grad_logits, labels, N, C, M))
-        return launch_rows_resident_step(prm, static_cast<cudaStream_t>(stream));
     return dispatch<KIND, true>(prm, dtype, true, static_cast<cudaStream_t>(stream));
 }
 
@@ -2921,6 +2423,24 @@ __global__ void __launch_bounds__(256) count_valid_kernel(const int64_t *labels,
 }
 
 }  // namespace
+
+bool short_rows_eligible(size_t es, const void *logits, const void *io, const void *labels, int64_t N, int64_t C,
+                         int64_t M) {
+    if (!(M == 1 && N >= 1 && C >= 1 && C <= kShortRowsMaxC && aligned16(logits) && aligned16(io))) return false;
+    const int64_t ve = int64_t(16 / es);
+    return (C % ve == 0 && C >= kVecMinC) || aligned16(labels);    // (rows_vec_kernel loads labels one by one)
+}
+
+int launch_rows_lsr_fwd(int dtype, const SoftmaxParams &prm, cudaStream_t stream);
+int launch_rows_lsr_bwd(int dtype, const SoftmaxParams &prm, cudaStream_t stream);
+int launch_rows_lmargin_fwd(int dtype, const SoftmaxParams &prm, cudaStream_t stream);
+int launch_rows_lmargin_bwd(int dtype, const SoftmaxParams &prm, cudaStream_t stream);
+
+int launch_short_rows(int kind, bool bwd, int dtype, const SoftmaxParams &prm, cudaStream_t stream) {
+    if (kind == kLSR) return bwd ? launch_rows_lsr_bwd(dtype, prm, stream) : launch_rows_lsr_fwd(dtype, prm, stream);
+    return bwd ? launch_rows_lmargin_bwd(dtype, prm, stream) : launch_rows_lmargin_fwd(dtype, prm, stream);
+}
+
 }  // namespace b200
 
 using namespace b200;

@@ -1,0 +1,49 @@
+"""Row layouts (M == 1): the lengths at which the row kernels change their walk, their lanes per row or
+their register budget, with remainders, against the oracle in 64 bits."""
+import pytest
+import torch
+
+from oracle import losses as O
+
+pytestmark = pytest.mark.gpu
+
+# classes: whole vectors / pairs / odd; 40 channels a lane at most, 256 and 2048 as bounds of the warp-by-row form
+CLASSES = [2, 3, 4, 8, 19, 20, 32, 40, 41, 42, 80, 81, 150, 160, 162, 255, 256, 257, 513, 1000, 1023, 1024, 1028, 1280,
+           1284, 1536, 1766, 2046, 2047, 2048]
+# float32: sums of at most 2048 terms in a tree of packed adds and an approximate exponential of 2^-21;
+# 16 bits: the result is rounded once (half 2^-11, bfloat16 2^-8 of the element)
+TOL = {torch.float32: 3e-6, torch.float16: 1e-3, torch.bfloat16: 4e-3}
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("kind", ["lsr", "lmargin"])
+@pytest.mark.parametrize("rows", [1, 67, 2500])
+def test_rows_against_64_bits(rows, kind, dtype):
+    import pytorch_loss as P
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    for c in CLASSES:
+        x = (torch.randn(rows, c, generator=g, device="cuda") * 2).to(dtype)
+        y = torch.randint(0, c, (rows,), generator=g, device="cuda")
+        y[1::7] = -100
+        up = torch.rand(rows, generator=g, device="cuda").to(dtype) + 0.5
+        for reduction in ("none", "sum"):
+            if kind == "lsr":
+                crit = P.LabelSmoothSoftmaxCEV3(0.1, reduction, -100)
+                want, want_grad = O.label_smooth_ce(x, y, 0.1, -100, reduction, torch.float64)
+            else:
+                crit = P.LargeMarginSoftmaxV3(0.3, reduction, -100)
+                want, want_grad = O.large_margin_softmax(x, y, 0.3, -100, reduction, torch.float64)
+            leaf = x.clone().requires_grad_(True)
+            loss = crit(leaf, y)
+            grad, = torch.autograd.grad(loss, leaf, up if reduction == "none" else None)
+            with torch.no_grad():
+                alone = crit(x, y)
+            if reduction == "none":
+                want_grad = want_grad * up.double().unsqueeze(1)
+            tol_loss = TOL[dtype] if reduction == "none" else TOL[torch.float32]
+            what = "%s c=%d %s %s" % (kind, c, dtype, reduction)
+            assert float((loss.detach().double() - want).norm()) <= tol_loss * float(want.norm()) + 1e-6, what
+            assert float((alone.double() - want).norm()) <= tol_loss * float(want.norm()) + 1e-6, what
+            # (bfloat16 target and off-target parts are rounded once each, and their sum in the upstream product)
+            assert float((grad.double() - want_grad).norm()) <= 2 * TOL[dtype] * float(want_grad.norm()) + 1e-6, what
+            assert not bool(grad[y == -100].any()), what
