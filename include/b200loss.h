@@ -369,6 +369,16 @@ int b200_taylor_softmax_forward(const void *feat, void *out, int64_t N, int64_t 
 int b200_taylor_softmax_backward(const void *grad, const void *feat, void *grad_feat, int64_t N,
                                  int64_t C, int64_t M, int dtype, int n, int use_log,
                                  void *stream);
+/* Taylor cross entropy as a training step: nll_loss of the log-Taylor softmax (order n) and its gradient
+ * from ONE read of the logits; `out`, `workspace`, `denom` (null: 'sum') and `flags` as for
+ * b200_pc_softmax_step; a label that is neither ignore_index nor a class stops the program with a
+ * device assertion, as torch's nll_loss does.  b200_taylor_ce_step_path: 1 when the layout has this step
+ * (float32, M > 1, at most 64 classes).  Backward: b200_rescale_gradient. */
+int b200_taylor_ce_step_path(const void *logits, const int64_t *labels, const void *grad_logits, int64_t N,
+                             int64_t C, int64_t M, int dtype);
+int b200_taylor_ce_step(const void *logits, const int64_t *labels, void *grad_logits, void *out,
+                        void *workspace, size_t workspace_bytes, const void *denom, int64_t N, int64_t C,
+                        int64_t M, int dtype, int64_t ignore_index, int n, int flags, void *stream);
 
 /* -------------------------------------------------- PC softmax cross entropy ---
  * Replaces the tensor-op chain of PCSoftmaxCrossEntropyV1 / PCSoftmaxCrossEntropyFunction

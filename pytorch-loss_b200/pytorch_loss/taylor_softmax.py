@@ -13,7 +13,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 import torch.amp as amp
 
-from . import _cabi
+from . import _cabi, _softmax_family
 
 
 def _view(feat, dim):
@@ -101,8 +101,58 @@ class LogTaylorSoftmaxV3(nn.Module):
         return taylor_softmax_v3(x, self.dim, self.n, use_log=True)
 
 
+def _ce_step(logits, labels, n, ignore_index, mean):
+    """The 'mean' / 'sum' training step in one pass over the logits: (record, final gradient), or None
+    when the layout has none."""
+    nn_, c, m = _cabi.split_shape(logits, labels)
+    logits, labels = logits.contiguous(), labels.contiguous()
+    lib = _cabi.load_library()
+    dev = logits.device
+    grads = torch.empty_like(logits)
+    if not lib.b200_taylor_ce_step_path(_cabi.ptr(logits), _cabi.ptr(labels), _cabi.ptr(grads), nn_, c, m, _cabi.F32):
+        return None
+    rec = _cabi.new_record(dev)
+    ws = _cabi.reduce_workspace(dev)
+    denom, flags = None, 0
+    if mean:       # (directly in front of the step's launch: it starts under the count's tail)
+        denom = _softmax_family.count_valid(labels, ignore_index)
+        flags = _cabi.STEP_AFTER_COUNT
+    with torch.cuda.device(dev):
+        _cabi.check(lib.b200_taylor_ce_step(
+            _cabi.ptr(logits), _cabi.ptr(labels), _cabi.ptr(grads), _cabi.ptr(rec), _cabi.ptr(ws), ws.numel(),
+            None if denom is None else _cabi._vp(denom.data_ptr()), nn_, c, m, _cabi.F32, int(ignore_index), int(n),
+            flags, _cabi.stream_ptr(dev)))
+    return rec, grads
+
+
+class _TaylorCEFunc(torch.autograd.Function):
+    """nll_loss of the log-Taylor softmax as one kernel for loss and gradient; backward multiplies by
+    the upstream gradient (a kernel that leaves at once when that is 1)."""
+
+    @staticmethod
+    @amp.custom_fwd(cast_inputs=torch.float32, device_type='cuda')
+    def forward(ctx, logits, labels, n, ignore_index, mean):
+        rec, ctx.grads = _ce_step(logits, labels, n, ignore_index, mean)
+        ctx.vars = logits, labels, n, ignore_index, mean
+        return rec[4] if mean else rec[5]
+
+    @staticmethod
+    @amp.custom_bwd(device_type='cuda')
+    def backward(ctx, grad_output):
+        grads, ctx.grads = ctx.grads, None
+        if grads is None:                     # a second trip through the graph: the first scaled them in place
+            _, grads = _ce_step(*ctx.vars)
+        g = grad_output.to(torch.float32).reshape(-1)[:1].contiguous()
+        with torch.cuda.device(grads.device):
+            _cabi.check(_cabi.load_library().b200_rescale_gradient(
+                _cabi.ptr(grads), _cabi.ptr(g), None, grads.numel(), _cabi.F32, _cabi.stream_ptr(grads.device)))
+        return grads, None, None, None, None
+
+
 class TaylorCrossEntropyLossV3(nn.Module):
-    """nll_loss of the log-Taylor softmax over dim 1 (reference :175-198)."""
+    """nll_loss of the log-Taylor softmax over dim 1 (reference :175-198).  Images of up to 64 classes
+    ('mean' / 'sum', float32 logits or autocast, a gradient to produce) run loss and gradient as one
+    kernel; everything else goes through the activation and torch's nll_loss."""
 
     def __init__(self, n=2, ignore_index=-1, reduction='mean'):
         super().__init__()
@@ -111,6 +161,22 @@ class TaylorCrossEntropyLossV3(nn.Module):
         self.reduction = reduction
         self.ignore_index = ignore_index
 
+    def _fused(self, logits, labels):
+        act = self.taylor_softmax
+        return (self.reduction in ('mean', 'sum') and type(act) is LogTaylorSoftmaxV3 and act.dim == 1 and
+                2 <= act.n <= 16 and act.n % 2 == 0 and
+                not (act._forward_hooks or act._forward_pre_hooks or act._backward_hooks or act._backward_pre_hooks) and
+                logits.is_cuda and logits.requires_grad and torch.is_grad_enabled() and
+                (logits.dtype == torch.float32 or
+                 (torch.is_autocast_enabled('cuda') and logits.dtype in (torch.float16, torch.bfloat16))) and
+                3 <= logits.dim() and logits.size(1) <= 64 and logits.numel() > 0 and
+                logits.numel() // (logits.size(0) * logits.size(1)) > 1 and
+                logits[0].numel() < 2 ** 31 and
+                labels.device == logits.device and labels.dtype == torch.int64 and
+                labels.shape == logits.shape[:1] + logits.shape[2:])
+
     def forward(self, logits, labels):
+        if self._fused(logits, labels):
+            return _TaylorCEFunc.apply(logits, labels, self.taylor_softmax.n, self.ignore_index, self.reduction == 'mean')
         log_probs = self.taylor_softmax(logits)
         return F.nll_loss(log_probs, labels, reduction=self.reduction, ignore_index=self.ignore_index)

@@ -1,12 +1,13 @@
 """Taylor softmax / log-Taylor softmax / Taylor cross entropy (CUDA, through the C ABI) against
 the CPU oracle and the golden file made from the reference's V1 functions."""
+import math
 import os
 
 import numpy as np
 import pytest
 import torch
 
-from helpers import labels_with_ignores
+from helpers import assert_grad_close, assert_loss_close, labels_with_ignores
 
 pytestmark = pytest.mark.gpu
 
@@ -86,3 +87,30 @@ def test_fp16_autocast_noncontiguous_empty_and_errors():
         P.taylor_softmax_v3(x, 1, 4)                       # CPU tensor: gpu only
     with pytest.raises(RuntimeError):
         P.TaylorSoftmaxFunc.apply(x.cuda(), 1, 18, False)  # order above the supported 16
+
+
+# class counts around the register budgets of the training step (8, 20, 24, 32, 40, 64, none above), pixel
+# counts that are even, odd and shorter than a warp
+@pytest.mark.parametrize("c", [1, 2, 8, 9, 20, 21, 25, 32, 33, 41, 64, 65])
+@pytest.mark.parametrize("shape", [(16, 18), (7, 9), (2,)])
+@pytest.mark.parametrize("order", [2, 8])
+def test_cross_entropy_step_against_64_bits(c, shape, order):
+    import pytorch_loss as P
+    g = torch.Generator().manual_seed(c * 100 + order)
+    x = torch.randn(3, c, *shape, generator=g)
+    y = torch.randint(0, c, (3,) + shape, generator=g)
+    y[torch.rand(y.shape, generator=g) < 0.2] = -1
+    y.view(-1)[0] = 0
+    for reduction in ("mean", "sum"):
+        ref = x.double().requires_grad_(True)
+        f = sum(ref.pow(i) / math.factorial(i) for i in range(order + 1))
+        want = torch.nn.functional.nll_loss((f / f.sum(1, keepdim=True)).log(), y, ignore_index=-1, reduction=reduction)
+        (want * 0.5).backward()
+        leaf = x.cuda().requires_grad_(True)
+        loss = P.TaylorCrossEntropyLossV3(order, -1, reduction)(leaf, y.cuda())
+        first, = torch.autograd.grad(loss, leaf, torch.tensor(0.5, device="cuda"), retain_graph=True)
+        first = first.clone()
+        again, = torch.autograd.grad(loss, leaf, torch.tensor(0.5, device="cuda"))
+        assert_loss_close(loss, want.float(), atol=1e-6)
+        assert_grad_close(first, ref.grad)
+        assert_grad_close(again, ref.grad)
