@@ -177,3 +177,38 @@ def test_unsupported_shapes_raise():
         P.LovaszSoftmaxV3()(torch.randn(1, 1100, 4, 4).cuda(), torch.zeros(1, 4, 4, dtype=torch.int64).cuda())
     with pytest.raises(ValueError):
         P.LovaszSoftmaxV3(process_group=True)
+
+
+# segments that are counted instead of sorted (from 262144 pixels and 4096 of a class on): pixel counts that are and
+# are not a multiple of 4, pruned and not, saturated pixels (the shared last bin), a class below the limit, and one
+# whose mistakes pile up in the first bin
+@pytest.mark.parametrize("shape,per_image", [((1, 3, 512, 512), True), ((2, 5, 513, 515), True), ((3, 4, 301, 293), False)])
+@pytest.mark.parametrize("kind", ["random", "trained", "saturated"])
+def test_counted_segments_against_64_bits(shape, per_image, kind):
+    import pytorch_loss as P
+    from oracle import losses as O
+    n, c, h, w = shape
+    g = torch.Generator().manual_seed(h)
+    x = torch.randn(shape, generator=g)
+    y = torch.randint(0, c, (n, h // 16 + 1, w // 16 + 1), generator=g).repeat_interleave(16, 1).repeat_interleave(16, 2)
+    y = y[:, :h, :w].contiguous()
+    y[y == c - 1] = 0                                           # the last class: 64 pixels an image only
+    y[:, :8, :8] = c - 1
+    if kind != "random":
+        lead = torch.rand((n, 1, h, w), generator=g) * (12 if kind == "trained" else 60) + 3
+        other = torch.randint(0, c, (n, h, w), generator=g)
+        wrong = torch.rand((n, h, w), generator=g) < 0.04
+        x.scatter_add_(1, torch.where(wrong, other, y).unsqueeze(1), lead)
+    y[torch.rand(y.shape, generator=g) < 0.03] = 255
+    want, want_grad = O.lovasz_softmax(x, y, 255, "sum", per_image=per_image, dtype=torch.float64)
+    leaf = x.cuda().requires_grad_(True)
+    loss = P.LovaszSoftmaxV3("sum", 255, per_image=per_image)(leaf, y.cuda())
+    grad, = torch.autograd.grad(loss, leaf)
+    assert_loss_close(loss, want, rtol=2e-6)                    # sums of fp32 terms; the order inside a bin cancels
+    # errors that agree to 2^-13 (counted) or in their float32 rounding (the 64-pixel class, sorted) change places:
+    # a step of dJ, at most 1/4096^2 of the one and 1/64^2 of the other, for few of the pixels
+    assert float((grad.double().cpu() - want_grad).abs().max()) <= 1.0 / 64 ** 2
+    # (swaps in the 64-pixel class, whose steps are the largest, alone make up 6e-5 of the norm in float32)
+    assert float((grad.double().cpu() - want_grad).norm()) <= 2e-4 * float(want_grad.norm())
+    again = P.LovaszSoftmaxV3("sum", 255, per_image=per_image)(leaf, y.cuda())
+    assert torch.equal(torch.autograd.grad(again, leaf)[0], grad) and torch.equal(again, loss)
