@@ -818,7 +818,9 @@ int launch_rows_short(SoftmaxParams prm, int tpr, cudaStream_t stream) {
 
 template <typename T, int KIND, bool BWD> int launch_rows_typed(const SoftmaxParams &prm, cudaStream_t stream) {
     constexpr int VE = 16 / int(sizeof(T));
-    if (prm.C % VE == 0 && prm.C >= kVecMinC) return launch_rows_vec<T, KIND, BWD>(prm, stream);
+    // (labels that do not start on 16 bytes cannot be copied in bulk)
+    if (prm.C % VE == 0 && (prm.C >= kVecMinC || (prm.C >= 16 * VE && !aligned16(prm.labels))))
+        return launch_rows_vec<T, KIND, BWD>(prm, stream);
     // lanes per row: the fewest that keep a lane's share within 20 pairs (what a row costs besides its
     // elements is paid by every one of its lanes)
     int tpr = 1;

@@ -2428,7 +2428,7 @@ bool short_rows_eligible(size_t es, const void *logits, const void *io, const vo
                          int64_t M) {
     if (!(M == 1 && N >= 1 && C >= 1 && C <= kShortRowsMaxC && aligned16(logits) && aligned16(io))) return false;
     const int64_t ve = int64_t(16 / es);
-    return (C % ve == 0 && C >= kVecMinC) || aligned16(labels);    // (rows_vec_kernel loads labels one by one)
+    return (C % ve == 0 && C >= 16 * ve) || aligned16(labels);    // (rows_vec_kernel loads labels one by one)
 }
 
 int launch_rows_lsr_fwd(int dtype, const SoftmaxParams &prm, cudaStream_t stream);

@@ -47,3 +47,21 @@ def test_rows_against_64_bits(rows, kind, dtype):
             # (bfloat16 target and off-target parts are rounded once each, and their sum in the upstream product)
             assert float((grad.double() - want_grad).norm()) <= 2 * TOL[dtype] * float(want_grad.norm()) + 1e-6, what
             assert not bool(grad[y == -100].any()), what
+
+
+@pytest.mark.parametrize("c", [64, 128, 252, 256])
+def test_rows_with_labels_on_8_bytes(c):
+    """Labels that do not start on 16 bytes (a slice) cannot be copied in bulk: the fused step is still there."""
+    import pytorch_loss as P
+    from pytorch_loss import _cabi
+    g = torch.Generator(device="cuda").manual_seed(c)
+    x = torch.randn(300, c, generator=g, device="cuda")
+    y = torch.randint(0, c, (301,), generator=g, device="cuda")[1:]
+    assert y.data_ptr() % 16 == 8
+    assert _cabi.load_library().b200_softmax_fused_step_path(x.data_ptr(), y.data_ptr(), x.data_ptr(), 300, c, 1, _cabi.F32)
+    want, want_grad = O.label_smooth_ce(x, y, 0.1, -100, "mean", torch.float64)
+    leaf = x.clone().requires_grad_(True)
+    loss = P.LabelSmoothSoftmaxCEV3(0.1, "mean", -100)(leaf, y)
+    grad, = torch.autograd.grad(loss, leaf)
+    assert abs(float(loss) - float(want)) <= 3e-6 * float(want)
+    assert float((grad.double() - want_grad).norm()) <= 6e-6 * float(want_grad.norm())
