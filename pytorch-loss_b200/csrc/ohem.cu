@@ -229,6 +229,76 @@ ohem_score_kernel(const T *__restrict__ logits, const int64_t *__restrict__ labe
     finish_pass(sh, ghist, st, 0, 20, k_first, thresh_bits);
 }
 
+// The same for few classes (float32): a thread keeps all channels of VEC adjacent pixels (2: M even, 8-byte
+// aligned; 1: any M) in registers, every load in flight before the first is used, one exponential per
+// element.  Bound by HBM (the chunked walk above keeps 8 loads in flight and rescales its sums):
+// [8, 19, 769, 769] 167 -> 91 us.
+template <int CMAX, int VEC>
+__global__ void __launch_bounds__(kOhemThreads, CMAX * VEC <= 20 ? 5 : CMAX * VEC <= 40 ? 3 : 2)
+ohem_score_resident_kernel(const float *__restrict__ logits, const int64_t *__restrict__ labels, float *__restrict__ scores,
+                           uint32_t *__restrict__ ghist, OhemState *st, int64_t N, int C, int64_t M64, int64_t ignore,
+                           uint32_t k_first, uint32_t thresh_bits) {
+    __shared__ uint32_t sh[kBinsPerPass];
+    for (int b = threadIdx.x; b < kBinsPerPass; b += kOhemThreads) sh[b] = 0u;
+    __syncthreads();
+    const int M = int(M64);                                  // C * M < 2^31 (host check): 32-bit channel offsets
+    const int64_t groups_per_image = M64 / VEC;
+    const int64_t groups = N * groups_per_image;
+    const int64_t stride = int64_t(gridDim.x) * kOhemThreads;
+    // every lane of a warp runs the same number of iterations (the histogram votes are warp-wide)
+    const int64_t rounds = (groups + stride - 1) / stride;
+    for (int64_t it = 0; it < rounds; ++it) {
+        const int64_t gidx = it * stride + int64_t(blockIdx.x) * kOhemThreads + threadIdx.x;
+        const bool live = gidx < groups;
+        float sc[VEC];
+        if (live) {
+            const int64_t n = gidx / groups_per_image, m0 = (gidx % groups_per_image) * VEC;
+            const float *col = logits + n * C * M64 + m0;
+            float x[CMAX][VEC];
+#pragma unroll
+            for (int j = 0; j < CMAX; ++j) {
+#pragma unroll
+                for (int v = 0; v < VEC; ++v) x[j][v] = -FLT_MAX;
+                if (j < C) {
+                    if constexpr (VEC == 2) {
+                        const float2 f = __ldcs(reinterpret_cast<const float2 *>(col + j * M));
+                        x[j][0] = f.x;
+                        x[j][1] = f.y;
+                    } else {
+                        x[j][0] = __ldcs(col + j * M);
+                    }
+                }
+            }
+#pragma unroll
+            for (int v = 0; v < VEC; ++v) {
+                const int64_t l = __ldg(labels + n * M64 + m0 + v);
+                // -1: ignored, -2: outside [0, C) (scores 0: counts as hard)
+                const int lb = l == ignore ? -1 : ((l >= 0 && l < C) ? int(l) : -2);
+                float mx = -FLT_MAX, xl = -FLT_MAX, sum = 0.f;
+#pragma unroll
+                for (int j = 0; j < CMAX; ++j) {
+                    mx = fmaxf(mx, x[j][v]);
+                    if (j == lb) xl = x[j][v];
+                }
+                const float off = -mx * kOhemLog2e;
+#pragma unroll
+                for (int j = 0; j < CMAX; ++j) {
+                    const float e = exp2f(fmaf(x[j][v], kOhemLog2e, off));
+                    if (j < C) sum += e;
+                }
+                sc[v] = lb == -1 ? 1.f : __fdividef(exp2f((xl - mx) * kOhemLog2e), sum);
+                scores[n * M64 + m0 + v] = sc[v];
+            }
+        }
+#pragma unroll
+        for (int v = 0; v < VEC; ++v) {
+            const uint32_t bin = min(__float_as_uint(live ? sc[v] : 0.f) >> 20, uint32_t(kBinsPerPass - 1));
+            hist_add(sh, bin, live);
+        }
+    }
+    finish_pass(sh, ghist, st, 0, 20, k_first, thresh_bits);
+}
+
 // Histogram of the next digit over the scores that match the prefix found so far.
 __global__ void __launch_bounds__(kOhemThreads)
 ohem_hist_kernel(const float *__restrict__ scores, uint32_t *__restrict__ ghist, OhemState *st, int64_t P, int pass,
@@ -349,7 +419,26 @@ extern "C" int b200_ohem_label(const void *logits, const int64_t *labels, int64_
     const int64_t cap = int64_t(sm_count()) * 8;
     if (grid > cap) grid = cap;
     const int Ci = int(C);
-    if (vec4)
+    const bool pairs = M % 2 == 0 && (reinterpret_cast<uintptr_t>(logits) & 7u) == 0;
+    if (dtype == B200_F32 && C * M < (int64_t(1) << 31) && C <= (pairs ? 32 : 64)) {
+        const int64_t rgroups = pairs ? P / 2 : P;
+        auto go = [&](auto kern, int per_sm) {               // all blocks resident: one histogram flush per block
+            int64_t rgrid = (rgroups + kOhemThreads - 1) / kOhemThreads;
+            if (rgrid > int64_t(sm_count()) * per_sm) rgrid = int64_t(sm_count()) * per_sm;
+            kern<<<unsigned(rgrid), kOhemThreads, 0, s>>>(static_cast<const float *>(logits), labels, w.scores, w.hist, w.state,
+                                                          N, Ci, M, ignore_index, k_first, thresh_bits);
+        };
+        if (pairs) {
+            if (C <= 8) go(ohem_score_resident_kernel<8, 2>, 5);
+            else if (C <= 20) go(ohem_score_resident_kernel<20, 2>, 3);
+            else go(ohem_score_resident_kernel<32, 2>, 2);
+        } else {
+            if (C <= 8) go(ohem_score_resident_kernel<8, 1>, 5);
+            else if (C <= 20) go(ohem_score_resident_kernel<20, 1>, 5);
+            else if (C <= 40) go(ohem_score_resident_kernel<40, 1>, 3);
+            else go(ohem_score_resident_kernel<64, 1>, 2);
+        }
+    } else if (vec4)
         ohem_score_kernel<float, 4><<<unsigned(grid), kOhemThreads, 0, s>>>(
             static_cast<const float *>(logits), labels, w.scores, w.hist, w.state, N, Ci, M, ignore_index, k_first, thresh_bits);
     else if (dtype == B200_F32)

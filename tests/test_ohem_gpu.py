@@ -123,3 +123,21 @@ def test_golden_from_reference_cuda(golden_dir):
         want = torch.from_numpy(z[f"c{i}_new_labels"])
         got = ohem_cpp.score_ohem_label(logits.cuda(), labels.cuda(), int(ign), float(thresh), int(n_min))
         assert torch.equal(got.cpu(), want), "case %d: %d labels differ" % (i, int((got.cpu() != want).sum()))
+
+
+# class counts around the score kernel's register budgets, even / odd / multiple-of-4 pixel counts
+@pytest.mark.parametrize("c", [1, 2, 8, 9, 20, 21, 32, 33, 40, 41, 64, 65])
+@pytest.mark.parametrize("hw", [(8, 12), (9, 14), (11, 13)])
+def test_scores_of_every_class_count(c, hw):
+    from pytorch_loss.ohem_loss import score_ohem_label
+    from oracle import ohem as OH
+    g = torch.Generator().manual_seed(c * 31 + hw[0])
+    x = torch.randn(3, c, *hw, generator=g) * 2
+    y = labels_with_ignores(g, (3,) + hw, c, 255, 0.1)
+    for thresh, n_min in ((0.7, y.numel() // 16), (0.05, 40), (2.0, 0)):
+        want, scores = OH.score_ohem_label(x, y, 255, thresh, n_min)
+        got = score_ohem_label(x.cuda(), y.cuda(), 255, thresh, n_min).cpu()
+        # the float32 score that is kept last may tie with others: they all stay here
+        cut = max(thresh, float(scores.flatten().sort().values[max(n_min, 1) - 1]))
+        clear = (scores - cut).abs() > 1e-6
+        assert torch.equal(got[clear], want[clear])
