@@ -69,7 +69,7 @@ class Exchange:
         if p is None:
             return
         rec, ws, state, corr = p
-        with torch.cuda.device(self.device):
+        with _cabi.on_device(self.device):
             _cabi.check(_cabi.load_library().b200_exchange_finish(
                 _cabi.ptr(ws), _cabi.ptr(rec), _cabi.ptr(state), _cabi.ptr(corr), _cabi.stream_ptr(self.device)))
 
@@ -82,7 +82,7 @@ class Exchange:
         if ws is None:
             lib = _cabi.load_library()
             ws = torch.zeros(int(lib.b200_reduce_workspace_bytes()), dtype=torch.uint8, device=self.device)
-            with torch.cuda.device(self.device):
+            with _cabi.on_device(self.device):
                 _cabi.check(lib.b200_reduce_attach_exchange(_cabi.ptr(ws), _cabi.ptr(self.ctx),
                                                             _cabi.stream_ptr(self.device)))
             self._workspaces[stream.cuda_stream] = ws
@@ -149,7 +149,7 @@ def _build(group, device):
         torch.cuda.synchronize(device)
         raw = ctypes.create_string_buffer(64)
         offset = ctypes.c_uint64(0)
-        with torch.cuda.device(device):
+        with _cabi.on_device(device):
             _cabi.check(lib.b200_ipc_export(_cabi.ptr(local), raw, ctypes.byref(offset)))
         handle = (bytes(raw.raw), int(offset.value))
     except Exception:                      # noqa: BLE001  any failure -> collective fallback, decided below
@@ -159,7 +159,7 @@ def _build(group, device):
     peers, exchange = {}, None
     if ok and all(h[0] for h in handles):
         try:
-            with torch.cuda.device(device):            # the handle must be opened with MY device current
+            with _cabi.on_device(device):            # the handle must be opened with MY device current
                 for p, (_, (raw_bytes, off)) in enumerate(handles):
                     if p != rank:
                         mapped = ctypes.c_void_p(0)

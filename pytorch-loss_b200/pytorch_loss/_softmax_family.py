@@ -53,7 +53,7 @@ def forward_per_pixel(kind, logits, labels, ignore_index, hyper, want_stats=Fals
     if want_stats and n * m > 0 and lib.b200_softmax_stats_path(_cabi.ptr(logits), _cabi.ptr(labels), None,
                                                                 n, c, m, dt):
         stats = torch.empty((n * m, 4), dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
+    with _cabi.on_device(dev):
         if stats is not None:
             _cabi.check(getattr(lib, _ENTRY_EX[kind][0])(
                 _cabi.ptr(logits), _cabi.ptr(labels), _cabi.ptr(losses), None, None, 0, _cabi.ptr(stats),
@@ -80,7 +80,7 @@ def forward_reduced(kind, logits, labels, ignore_index, hyper, want_losses=False
     if want_stats and n * m > 0 and lib.b200_softmax_stats_path(_cabi.ptr(logits), _cabi.ptr(labels), None,
                                                                 n, c, m, dt):
         stats = torch.empty((n * m, 4), dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
+    with _cabi.on_device(dev):
         if stats is not None:
             _cabi.check(getattr(lib, _ENTRY_EX[kind][0])(
                 _cabi.ptr(logits), _cabi.ptr(labels), _cabi.ptr(losses), _cabi.ptr(rec), _cabi.ptr(ws),
@@ -110,7 +110,7 @@ def backward(kind, logits, labels, grad_output, denom, ignore_index, hyper, stat
         if mode == 2:
             g = g.to(logits.dtype)
     dptr = None if denom is None else _cabi._vp(denom.data_ptr())
-    with torch.cuda.device(dev):
+    with _cabi.on_device(dev):
         if stats is not None:
             _cabi.check(getattr(lib, _ENTRY_EX[kind][1])(
                 _cabi.ptr(logits), _cabi.ptr(labels), _cabi.ptr(stats), _cabi.ptr(g), mode, dptr, _cabi.ptr(grads),
@@ -138,10 +138,10 @@ def count_valid(labels, ignore_index, exchange=None):
     labels = labels.contiguous()
     ws = exchange.workspace() if exchange is not None else _cabi.reduce_workspace(dev)
     cnt = _cabi.new_record(dev)
-    with torch.cuda.device(dev):
+    with _cabi.on_device(dev):
         _cabi.check(lib.b200_count_valid(_cabi.ptr(labels), labels.numel(), int(ignore_index), _cabi.ptr(cnt),
                                          _cabi.ptr(ws), ws.numel(), _cabi.stream_ptr(dev)))
-    return cnt[:4].view(torch.float64)[1:]
+    return _cabi.record_count(cnt)
 
 
 def fused_step(kind, logits, labels, ignore_index, hyper, mean, exchange, denom=None):
@@ -161,16 +161,19 @@ def fused_step(kind, logits, labels, ignore_index, hyper, mean, exchange, denom=
     # across GPUs the kernel only posts its sums; backward's rescale kernel collects the peers'
     # (or whatever reads the loss first, see _p2p.DeferredLoss)
     flags = _cabi.STEP_DEFER if (exchange is not None and _p2p.defer_enabled()) else 0
-    if mean and denom is None:
-        # everything the step needs is allocated by now: the label count is the operation directly
-        # in front of the step's kernel, which may then start under the count's tail
-        denom = count_valid(labels, ignore_index, exchange)
-        flags |= _cabi.STEP_AFTER_COUNT
-    with torch.cuda.device(dev):
+    lp, wp, wn = _cabi.ptr(labels), _cabi.ptr(ws), ws.numel()
+    denom_ptr = None if denom is None or not mean else denom.data_ptr()
+    with _cabi.on_device(dev):
+        if mean and denom is None:
+            # everything the step needs is allocated by now: the label count is the operation directly
+            # in front of the step's kernel, which may then start under the count's tail
+            count = _cabi.new_record(dev)
+            denom_ptr = count.data_ptr() + _cabi.RECORD_COUNT
+            _cabi.check(lib.b200_count_valid(lp, labels.numel(), int(ignore_index), count.data_ptr(), wp, wn, st))
+            flags |= _cabi.STEP_AFTER_COUNT
         _cabi.check(getattr(lib, _ENTRY_FUSED[kind])(
-            _cabi.ptr(logits), _cabi.ptr(labels), _cabi.ptr(grads), _cabi.ptr(rec), _cabi.ptr(ws), ws.numel(),
-            None if not mean else _cabi._vp(denom.data_ptr()), n, c, m, dt, int(ignore_index), float(hyper),
-            flags, st))
+            _cabi.ptr(logits), lp, _cabi.ptr(grads), _cabi.ptr(rec), wp, wn,
+            denom_ptr, n, c, m, dt, int(ignore_index), float(hyper), flags, st))
     defer = flags & _cabi.STEP_DEFER
     if defer:
         exchange.defer(rec, ws)
@@ -203,8 +206,7 @@ class ReducedLossFunc(torch.autograd.Function):
                 rec, grads, logits, labels = step
                 ctx.fused = grads
                 ctx.deferred = (exchange, rec) if (exchange is not None and exchange.pending is not None) else None
-                ctx.variables = (logits, labels, kind, hyper, ignore_index,
-                                 (rec[:4].view(torch.float64)[1:] if mean else None), None)
+                ctx.variables = logits, labels, kind, hyper, ignore_index, (rec if mean else None), None
                 return rec[4] if mean else rec[5]
         if exchange is not None and mean:
             _cabi.require_cuda(logits, labels)
@@ -222,17 +224,16 @@ class ReducedLossFunc(torch.autograd.Function):
         ctx.variables = logits, labels, kind, hyper, ignore_index, (sum_count[1:] if mean else None), stats
         return loss
 
-    @staticmethod
-    @amp.custom_bwd(device_type='cuda')
+    @staticmethod                             # (nothing in here depends on autocast)
     def backward(ctx, grad_output):
         logits, labels, kind, hyper, ignore_index, denom, stats = ctx.variables
         if ctx.fused is not None:
             # first trip through the graph: the gradient is there, times the upstream gradient
             grads, ctx.fused = ctx.fused, None
-            g = grad_output.to(torch.float32).reshape(-1)[:1].contiguous()
+            g = _cabi.scalar_gradient(grad_output)
             lib = _cabi.load_library()
             pending = ctx.deferred[0].take_pending(ctx.deferred[1]) if ctx.deferred else None
-            with torch.cuda.device(logits.device):
+            with _cabi.on_device(logits.device):
                 if pending is not None:
                     rec, ws, _, _ = pending
                     _cabi.check(lib.b200_rescale_gradient_finish(
@@ -243,6 +244,8 @@ class ReducedLossFunc(torch.autograd.Function):
                         _cabi.ptr(grads), _cabi.ptr(g), None, grads.numel(), _cabi.dtype_code(grads),
                         _cabi.stream_ptr(logits.device)))
             return grads, None, None, None, None, None, None
+        if denom is not None and denom.dtype != torch.float64:      # (the fused step left its whole record)
+            denom = _cabi.record_count(denom)
         grads = backward(kind, logits, labels, grad_output, denom, ignore_index, hyper, stats)
         return grads, None, None, None, None, None, None
 

@@ -47,7 +47,7 @@ def _focal_backward(logits, labels, grad_output, denom, alpha, gamma):
             g = g.to(logits.dtype)
             if not logits.is_contiguous():       # elementwise kernel: same memory layout as the logits
                 g = torch.empty_like(logits).copy_(g)
-    with torch.cuda.device(dev):
+    with _cabi.on_device(dev):
         _cabi.check(lib.b200_focal_backward(
             _cabi.ptr(logits), _cabi.ptr(labels), _cabi.ptr(g), mode,
             None if denom is None else _cabi._vp(denom.data_ptr()),
@@ -66,7 +66,7 @@ class FocalSigmoidLossFuncV3(torch.autograd.Function):
         dev, logits, labels, dt = _prep(logits, labels)
         lib = _cabi.load_library()
         losses = torch.empty_like(logits)
-        with torch.cuda.device(dev):
+        with _cabi.on_device(dev):
             _cabi.check(lib.b200_focal_forward(
                 _cabi.ptr(logits), _cabi.ptr(labels), _cabi.ptr(losses), None, None, 0,
                 logits.numel(), dt, float(gamma), float(alpha), _cabi.stream_ptr(dev)))
@@ -91,7 +91,7 @@ class FocalSigmoidLossFuncV3FB(torch.autograd.Function):
         lib = _cabi.load_library()
         losses = torch.empty_like(logits)
         grads = torch.empty_like(logits)
-        with torch.cuda.device(dev):
+        with _cabi.on_device(dev):
             _cabi.check(lib.b200_focal_forward_backward(
                 _cabi.ptr(logits), _cabi.ptr(labels), _cabi.ptr(losses), _cabi.ptr(grads),
                 logits.numel(), dt, float(gamma), float(alpha), _cabi.stream_ptr(dev)))
@@ -129,7 +129,7 @@ class _FocalReducedFunc(torch.autograd.Function):
         scale = 1.0
         correction = None
         st = _cabi.stream_ptr(dev)
-        with torch.cuda.device(dev):
+        with _cabi.on_device(dev):
             if mean and exchange is not None:
                 # The gradients need the GLOBAL element count.  A module keeps the count its
                 # previous call found on the device and divides by that; the kernel checks it
@@ -167,7 +167,7 @@ class _FocalReducedFunc(torch.autograd.Function):
                 exchange.defer(rec, ws, predicted if correction is not None else None, correction)
         ctx.deferred = (exchange, rec) if defer else None
         ctx.fused = [grads, correction]      # handed out by the first backward
-        ctx.variables = logits, labels, alpha, gamma, (rec[:4].view(torch.float64)[1:] if mean else None)
+        ctx.variables = logits, labels, alpha, gamma, (rec if mean else None)
         return rec[4] if mean else rec[5]
 
     @staticmethod
@@ -184,7 +184,7 @@ class _FocalReducedFunc(torch.autograd.Function):
         rec = _cabi.new_record(dev)
         exchange = _p2p.get_exchange(group, dev)      # sums over the ranks inside the kernel, if possible
         ws = exchange.workspace() if exchange is not None else _cabi.reduce_workspace(dev)
-        with torch.cuda.device(dev):
+        with _cabi.on_device(dev):
             _cabi.check(lib.b200_focal_forward(
                 _cabi.ptr(logits), _cabi.ptr(labels), None, _cabi.ptr(rec), _cabi.ptr(ws),
                 ws.numel(), logits.numel(), dt, float(gamma), float(alpha), _cabi.stream_ptr(dev)))
@@ -199,17 +199,16 @@ class _FocalReducedFunc(torch.autograd.Function):
         ctx.variables = logits, labels, alpha, gamma, (sum_count[1:] if mean else None)
         return loss
 
-    @staticmethod
-    @amp.custom_bwd(device_type='cuda')
+    @staticmethod                             # (nothing in here depends on autocast)
     def backward(ctx, grad_output):
         logits, labels, alpha, gamma, denom = ctx.variables
         if ctx.fused:
             grads, correction = ctx.fused
             ctx.fused = None
-            g = grad_output.to(torch.float32).reshape(-1)[:1].contiguous()
+            g = _cabi.scalar_gradient(grad_output)
             lib = _cabi.load_library()
             pending = ctx.deferred[0].take_pending(ctx.deferred[1]) if ctx.deferred else None
-            with torch.cuda.device(logits.device):
+            with _cabi.on_device(logits.device):
                 if pending is not None:
                     rec, ws, state, _ = pending
                     _cabi.check(lib.b200_rescale_gradient_finish(
@@ -220,6 +219,8 @@ class _FocalReducedFunc(torch.autograd.Function):
                         _cabi.ptr(grads), _cabi.ptr(g), _cabi.ptr(correction), grads.numel(), _cabi.dtype_code(grads),
                         _cabi.stream_ptr(logits.device)))
             return grads, None, None, None, None, None, None
+        if denom is not None and denom.dtype != torch.float64:      # (the fused step left its whole record)
+            denom = _cabi.record_count(denom)
         grads = _focal_backward(logits, labels, grad_output, denom, alpha, gamma)
         return grads, None, None, None, None, None, None
 

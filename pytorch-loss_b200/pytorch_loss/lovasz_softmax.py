@@ -34,7 +34,7 @@ def lovasz_forward(logits, labels, ignore_index, per_image=False):
         return loss.zero_(), jacc, x, labels
     nbytes = int(lib.b200_lovasz_workspace_bytes(n, c, m, int(per_image)))
     ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
-    with torch.cuda.device(dev):
+    with _cabi.on_device(dev):
         _cabi.check(lib.b200_lovasz_forward(
             _cabi.ptr(x), _cabi.ptr(labels), _cabi.ptr(loss), _cabi.ptr(jacc), _cabi.ptr(ws), nbytes,
             n, c, m, _cabi.F32, int(ignore_index), int(per_image), _cabi.stream_ptr(dev)))
@@ -49,7 +49,7 @@ def lovasz_backward(grad, logits, labels, jacc, ignore_index, per_image=False):
     lib = _cabi.load_library()
     g = grad.to(torch.float32).expand((n, c) if per_image else (c,)).contiguous()
     grads = torch.empty_like(logits, dtype=torch.float32)
-    with torch.cuda.device(dev):
+    with _cabi.on_device(dev):
         _cabi.check(lib.b200_lovasz_backward(
             _cabi.ptr(g), _cabi.ptr(logits), _cabi.ptr(labels), _cabi.ptr(jacc.contiguous()),
             _cabi.ptr(grads), n, c, m, _cabi.F32, int(ignore_index), int(per_image),

@@ -37,7 +37,7 @@ def score_ohem_label(logits, labels, ignore_index, score_thresh, n_min):
     lib = _cabi.load_library()
     nbytes = int(lib.b200_ohem_workspace_bytes(n, m))
     ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
-    with torch.cuda.device(dev):
+    with _cabi.on_device(dev):
         _cabi.check(lib.b200_ohem_label(
             _cabi.ptr(x), _cabi.ptr(lb), _cabi.ptr(out), _cabi.ptr(ws), nbytes, n, c, m,
             _cabi.dtype_code(x), int(ignore_index), float(score_thresh), n_min, _cabi.stream_ptr(dev)))

@@ -35,7 +35,7 @@ def pc_softmax_ce(logits, labels, lb_proportion, ignore_index, want_grad=True, d
     w = _weights(lb_proportion, c, dev)
     losses = torch.empty(labels.shape, dtype=logits.dtype, device=dev)
     grads = torch.empty_like(logits) if want_grad else None
-    with torch.cuda.device(dev):
+    with _cabi.on_device(dev):
         _cabi.check(_cabi.load_library().b200_pc_softmax_ce_scaled(
             _cabi.ptr(logits), _cabi.ptr(labels), _cabi.ptr(w), _cabi.ptr(losses), _cabi.ptr(grads),
             None if denom is None else _cabi._vp(denom.data_ptr()),
@@ -45,8 +45,8 @@ def pc_softmax_ce(logits, labels, lb_proportion, ignore_index, want_grad=True, d
 
 def _rescale(grads, grad_output):
     """grads *= grad_output (a scalar) in place; the kernel leaves at once when it is 1."""
-    g = grad_output.to(torch.float32).reshape(-1)[:1].contiguous()
-    with torch.cuda.device(grads.device):
+    g = _cabi.scalar_gradient(grad_output)
+    with _cabi.on_device(grads.device):
         _cabi.check(_cabi.load_library().b200_rescale_gradient(
             _cabi.ptr(grads), _cabi.ptr(g), None, grads.numel(), _cabi.dtype_code(grads),
             _cabi.stream_ptr(grads.device)))
@@ -56,7 +56,7 @@ def _rescale(grads, grad_output):
 def pc_softmax_step(logits, labels, lb_proportion, ignore_index, mean):
     """The 'mean' / 'sum' training step in one pass over the logits (the label-smooth step's tile
     pipeline with the class weights inside the exponentials), or None when the layout has none.
-    Returns (record, final gradient, valid-pixel count or None)."""
+    Returns (record, final gradient, record of the valid-pixel count or None)."""
     dev = _cabi.require_cuda(logits, labels)
     n, c, m = _cabi.split_shape(logits, labels)
     if labels.dtype != torch.int64 or logits.dtype not in (torch.float32, torch.float16, torch.bfloat16):
@@ -70,16 +70,18 @@ def pc_softmax_step(logits, labels, lb_proportion, ignore_index, mean):
     w = _weights(lb_proportion, c, dev)
     rec = _cabi.new_record(dev)
     ws = _cabi.reduce_workspace(dev)
-    denom, flags = None, 0
-    if mean:       # (directly in front of the step's launch: it starts under the count's tail)
-        denom = _softmax_family.count_valid(labels, ignore_index)
-        flags = _cabi.STEP_AFTER_COUNT
-    with torch.cuda.device(dev):
+    denom, flags, count = None, 0, None
+    st, lp, wp, wn = _cabi.stream_ptr(dev), _cabi.ptr(labels), _cabi.ptr(ws), ws.numel()
+    with _cabi.on_device(dev):
+        if mean:       # (directly in front of the step's launch: it starts under the count's tail)
+            count = _cabi.new_record(dev)
+            denom = count.data_ptr() + _cabi.RECORD_COUNT
+            _cabi.check(lib.b200_count_valid(lp, labels.numel(), int(ignore_index), count.data_ptr(), wp, wn, st))
+            flags = _cabi.STEP_AFTER_COUNT
         _cabi.check(lib.b200_pc_softmax_step(
-            _cabi.ptr(logits), _cabi.ptr(labels), _cabi.ptr(w), _cabi.ptr(grads), _cabi.ptr(rec), _cabi.ptr(ws),
-            ws.numel(), None if denom is None else _cabi._vp(denom.data_ptr()), n, c, m, dt, int(ignore_index),
-            flags, _cabi.stream_ptr(dev)))
-    return rec, grads, denom
+            _cabi.ptr(logits), lp, _cabi.ptr(w), _cabi.ptr(grads), _cabi.ptr(rec), wp, wn, denom, n, c, m, dt,
+            int(ignore_index), flags, st))
+    return rec, grads, count
 
 
 class PCSoftmaxCrossEntropyFunction(torch.autograd.Function):
@@ -111,12 +113,13 @@ class PCSoftmaxCrossEntropyFunction(torch.autograd.Function):
             return losses.sum(dtype=torch.float32)
         return losses
 
-    @staticmethod
-    @amp.custom_bwd(device_type='cuda')
+    @staticmethod                             # (nothing in here depends on autocast)
     def backward(ctx, grad_output):
         logits, label, lb_proportion, ignore_index, reduction, n_valid = ctx.vars
         grads, ctx.grads = ctx.grads, None
         if grads is None:                     # a second trip through the graph: the first scaled them in place
+            if n_valid is not None and n_valid.dtype != torch.float64:      # (the fused step left its whole record)
+                n_valid = _cabi.record_count(n_valid)
             _, grads = pc_softmax_ce(logits, label, lb_proportion, ignore_index, True, n_valid)
         if reduction in ('mean', 'sum'):
             return _rescale(grads, grad_output), None, None, None, None

@@ -13,7 +13,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 import torch.amp as amp
 
-from . import _cabi, _softmax_family
+from . import _cabi
 
 
 def _view(feat, dim):
@@ -34,7 +34,7 @@ def taylor_softmax_forward(feat, dim, n, use_log):
     nn_, c, m, _ = _view(feat, int(dim))
     out = torch.empty_like(feat)
     lib = _cabi.load_library()
-    with torch.cuda.device(dev):
+    with _cabi.on_device(dev):
         _cabi.check(lib.b200_taylor_softmax_forward(
             _cabi.ptr(feat), _cabi.ptr(out), nn_, c, m, _cabi.dtype_code(feat), int(n), int(bool(use_log)),
             _cabi.stream_ptr(dev)))
@@ -49,7 +49,7 @@ def taylor_softmax_backward(grad, feat, dim, n, use_log):
     nn_, c, m, _ = _view(feat, int(dim))
     out = torch.empty_like(feat)
     lib = _cabi.load_library()
-    with torch.cuda.device(dev):
+    with _cabi.on_device(dev):
         _cabi.check(lib.b200_taylor_softmax_backward(
             _cabi.ptr(grad), _cabi.ptr(feat), _cabi.ptr(out), nn_, c, m, _cabi.dtype_code(feat), int(n),
             int(bool(use_log)), _cabi.stream_ptr(dev)))
@@ -114,14 +114,16 @@ def _ce_step(logits, labels, n, ignore_index, mean):
     rec = _cabi.new_record(dev)
     ws = _cabi.reduce_workspace(dev)
     denom, flags = None, 0
-    if mean:       # (directly in front of the step's launch: it starts under the count's tail)
-        denom = _softmax_family.count_valid(labels, ignore_index)
-        flags = _cabi.STEP_AFTER_COUNT
-    with torch.cuda.device(dev):
+    st, lp, wp, wn = _cabi.stream_ptr(dev), _cabi.ptr(labels), _cabi.ptr(ws), ws.numel()
+    with _cabi.on_device(dev):
+        if mean:       # (directly in front of the step's launch: it starts under the count's tail)
+            count = _cabi.new_record(dev)
+            denom = count.data_ptr() + _cabi.RECORD_COUNT
+            _cabi.check(lib.b200_count_valid(lp, labels.numel(), int(ignore_index), count.data_ptr(), wp, wn, st))
+            flags = _cabi.STEP_AFTER_COUNT
         _cabi.check(lib.b200_taylor_ce_step(
-            _cabi.ptr(logits), _cabi.ptr(labels), _cabi.ptr(grads), _cabi.ptr(rec), _cabi.ptr(ws), ws.numel(),
-            None if denom is None else _cabi._vp(denom.data_ptr()), nn_, c, m, _cabi.F32, int(ignore_index), int(n),
-            flags, _cabi.stream_ptr(dev)))
+            _cabi.ptr(logits), lp, _cabi.ptr(grads), _cabi.ptr(rec), wp, wn, denom, nn_, c, m, _cabi.F32,
+            int(ignore_index), int(n), flags, st))
     return rec, grads
 
 
@@ -136,14 +138,13 @@ class _TaylorCEFunc(torch.autograd.Function):
         ctx.vars = logits, labels, n, ignore_index, mean
         return rec[4] if mean else rec[5]
 
-    @staticmethod
-    @amp.custom_bwd(device_type='cuda')
+    @staticmethod                             # (nothing in here depends on autocast)
     def backward(ctx, grad_output):
         grads, ctx.grads = ctx.grads, None
         if grads is None:                     # a second trip through the graph: the first scaled them in place
             _, grads = _ce_step(*ctx.vars)
-        g = grad_output.to(torch.float32).reshape(-1)[:1].contiguous()
-        with torch.cuda.device(grads.device):
+        g = _cabi.scalar_gradient(grad_output)
+        with _cabi.on_device(grads.device):
             _cabi.check(_cabi.load_library().b200_rescale_gradient(
                 _cabi.ptr(grads), _cabi.ptr(g), None, grads.numel(), _cabi.F32, _cabi.stream_ptr(grads.device)))
         return grads, None, None, None, None
