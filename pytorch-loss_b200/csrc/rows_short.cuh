@@ -478,6 +478,8 @@ rows_short_kernel(const SoftmaxParams prm) {
                 }
             }
             if (!BWD) {
+                // (the stand-ins were plain stores: order them before the copy that refills the stage)
+                if (KIND == kLMargin) fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&bars.empty[s]);
             } else {

@@ -766,6 +766,8 @@ tile_pair_kernel(const SoftmaxParams prm, const __grid_constant__ CUtensorMap ma
                             }
                         }
                     }
+                    // (the target's place was written by plain stores: order them before the copy that refills the stage)
+                    fence_proxy_async_smem();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&bars.empty[s]);
                 } else {
@@ -988,6 +990,8 @@ tile_chunk_fwd_kernel(const SoftmaxParams prm, const __grid_constant__ CUtensorM
                     sde = upk2(psde);
                     sx = upk2(psx);
                 }
+                // (the target's stand-in was a plain store: order it before the copy that refills the stage)
+                if (KIND == kLMargin) fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&bars.empty[s]);
             }
@@ -1497,6 +1501,8 @@ rows_pipe_kernel(const SoftmaxParams prm) {
                             acc_cnt += 1.0;
                         }
                     }
+                    // (the target's place was written by plain stores: order them before the copy that refills the stage)
+                    fence_proxy_async_smem();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&bars.empty[s]);
                 } else {

@@ -306,3 +306,22 @@ def test_empty_batch_reduced(kind):
         loss.backward()
         assert x.grad.shape == x.shape
         assert torch.isnan(loss.detach()) if reduction == "mean" else float(loss.detach()) == 0.0
+
+
+# Forward large margin writes the target's place in a stage before the copy pipeline refills it: enough tiles, chunks or
+# rows that every stage is refilled several times (two-box tiles, channel chunks, a row per stage, short rows).  An
+# element of a later tile lost to such a write would show at one pixel.
+@pytest.mark.parametrize("shape,dtype", [((2, 19, 900, 700), torch.float32), ((1, 41, 800, 512), torch.float32),
+                                         ((2500, 3000), torch.float16), ((60001, 150), torch.float16),
+                                         ((90001, 19), torch.float32)], ids=str)
+def test_large_margin_forward_through_refilled_stages(shape, dtype):
+    from oracle import losses as O
+    import pytorch_loss as P
+    g = torch.Generator(device="cuda").manual_seed(shape[1])
+    x = torch.randn(shape, generator=g, device="cuda").mul_(2).to(dtype)
+    y = torch.randint(0, shape[1], shape[:1] + shape[2:], generator=g, device="cuda")
+    want = O.large_margin_softmax(x, y, 0.3, 255, "none", torch.float64)[0]
+    with torch.no_grad():
+        got = P.LargeMarginSoftmaxV3(0.3, "none", 255)(x, y).double()
+    # float32: exponentials and logarithm of 2^-21, sums of `c` terms; half: the loss is rounded once, 2^-11
+    assert float(((got - want).abs() - (1e-3 if dtype is torch.float16 else 4e-6) * want.abs()).max()) <= 4e-6
