@@ -277,16 +277,18 @@ rows_short_kernel(const SoftmaxParams prm) {
                 const bool owner = lbi >= 0 && (lunit & (TPR - 1)) == t;      // my walk visits the label's unit
                 float xl = 0.f, xd = 0.f;
                 if (lbi >= 0) xl = to_f32(rp[lbi]);
-                if constexpr (KIND == kLMargin) {
+                T dup{};
+                if (KIND == kLMargin && lbi >= 0) {
                     // the target's place holds another channel's logit during the sums
-                    if (lbi >= 0) {
-                        const T dup = rp[(lbi == 0 && C > 1) ? 1 : 0];
-                        xd = to_f32(dup);
-                        __syncwarp(row_mask);                         // all of the row's lanes hold x_lb by now
-                        if (owner) rp[lbi] = dup;
-                    } else {
-                        xl = kNegInf;
-                    }
+                    dup = rp[(lbi == 0 && C > 1) ? 1 : 0];
+                    xd = to_f32(dup);
+                }
+                // every lane of the row has read x_lb before its owner writes there: the stand-in now or the
+                // gradient later (shuffles in between do not order memory)
+                if (KIND == kLMargin || BWD) __syncwarp(row_mask);
+                if constexpr (KIND == kLMargin) {
+                    if (lbi < 0) xl = kNegInf;
+                    else if (owner) rp[lbi] = dup;
                 }
                 // a walk over my units: `w` is where it stands, `left` the units before a rotated one wraps
                 const int rot = MODE == kRotated ? rowl % cnt : 0;

@@ -65,3 +65,46 @@ def test_rows_with_labels_on_8_bytes(c):
     grad, = torch.autograd.grad(loss, leaf)
     assert abs(float(loss) - float(want)) <= 3e-6 * float(want)
     assert float((grad.double() - want_grad).norm()) <= 6e-6 * float(want_grad.norm())
+
+
+# Many rows: several groups of rows in a stage and stages refilled many times, one to four lanes a row with the
+# rotated walk, and (256 classes and more) warps that take several rows with the next one in flight.  Row counts are
+# odd, so that the last stage is ragged.  Compared row by row: one row taken from another one's stage would show.
+MANY = {300007: [2, 3, 19, 20, 21, 36, 40], 60001: [80, 150, 160, 162, 255], 20003: [256, 1000, 1024, 2047, 2048]}
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("kind", ["lsr", "lmargin"])
+@pytest.mark.parametrize("rows", MANY)
+def test_many_rows_against_64_bits(rows, kind, dtype):
+    import pytorch_loss as P
+    g = torch.Generator(device="cuda").manual_seed(rows + 1)
+    for c in MANY[rows]:
+        x = (torch.randn(rows, c, generator=g, device="cuda") * 2).to(dtype)
+        y = torch.randint(0, c, (rows,), generator=g, device="cuda")
+        y[torch.rand(rows, generator=g, device="cuda") < 0.1] = -100
+        up = torch.rand(rows, generator=g, device="cuda").to(dtype) + 0.5
+        valid = y != -100
+        oracle = (lambda: O.label_smooth_ce(x, y, 0.1, -100, "none", torch.float64)) if kind == "lsr" else \
+            (lambda: O.large_margin_softmax(x, y, 0.3, -100, "none", torch.float64))
+        want, want_grad = oracle()
+        # (half: a gradient divided by the number of rows has too few bits)
+        for reduction in ("none", "sum") if dtype is torch.float16 else ("none", "sum", "mean"):
+            crit = P.LabelSmoothSoftmaxCEV3(0.1, reduction, -100) if kind == "lsr" else \
+                P.LargeMarginSoftmaxV3(0.3, reduction, -100)
+            leaf = x.clone().requires_grad_(True)
+            loss = crit(leaf, y)
+            grad, = torch.autograd.grad(loss, leaf, up if reduction == "none" else None)
+            what = "%s c=%d %s %s" % (kind, c, dtype, reduction)
+            if reduction == "none":
+                scale = up.double().unsqueeze(1)
+                assert float(((loss.detach().double() - want).abs() - TOL[dtype] * want.abs()).max()) <= 4e-6, what
+            else:
+                scale = 1.0 / float(valid.sum()) if reduction == "mean" else 1.0
+                total = float(want.sum()) * scale
+                assert abs(float(loss.detach()) - total) <= 3e-6 * abs(total), what
+            ref = want_grad * scale
+            # a row's gradient: rounded once in 16 bits, twice where the upstream gradient comes in
+            err = (grad.double() - ref).norm(dim=1) - 2 * TOL[dtype] * ref.norm(dim=1)
+            assert float(err.max()) <= (1e-6 if reduction != "mean" else 1e-6 * scale), what
+            assert not bool(grad[~valid].any()), what
