@@ -900,8 +900,9 @@ sort_scan_kernel(uint32_t *__restrict__ hist, uint32_t *__restrict__ fghist,
 // sort tile, a scan per segment, and a stable compaction that also writes the dropped
 // elements' dJ (zero).  The sort then runs on the kept elements only (Lp per segment).
 
-// A block takes `per` consecutive tiles of one segment (grid ceil(T / per) x S): with many tiles, segments
-// that are binned and have nothing to do here cost fewer blocks (19 456 of them took 23 us to find out).
+// A block takes `per` consecutive tiles of one segment (a flat grid of S * ceil(T / per): there may be more segments
+// than gridDim.y can count): with many tiles, segments that are binned and have nothing to do here cost fewer
+// blocks (19 456 of them took 23 us to find out).
 
 // kept[seg][tile] = number of elements of the tile with (key >> 1) < limit;
 // fgkept[seg][tile] = number of foreground elements of the tile.
@@ -911,10 +912,10 @@ prune_count_kernel(const uint32_t *__restrict__ keys, const uint32_t *__restrict
                    uint32_t *__restrict__ kept, uint32_t *__restrict__ fgkept, int64_t L, int64_t T, int prune,
                    int per) {
     __shared__ uint32_t wsum[kSortWarps], wfg[kSortWarps];
-    const int64_t seg = blockIdx.y;
+    const int64_t runs = (T + per - 1) / per, seg = blockIdx.x / runs, first = (blockIdx.x % runs) * per;
     if (__ldg(seg_flags + seg) & kSegFlagBinned) return;
     const uint32_t limit = prune_limit(maxfg, minkey, seg, prune);
-  for (int64_t tile = int64_t(blockIdx.x) * per; tile < T && tile < (int64_t(blockIdx.x) + 1) * per; ++tile) {
+  for (int64_t tile = first; tile < T && tile < first + per; ++tile) {
     const int64_t t0 = tile * kSortTile;
     const int n = int(L - t0 < kSortTile ? L - t0 : kSortTile);
     const uint32_t *src = keys + seg * L + t0;
@@ -1101,17 +1102,18 @@ class_count_kernel(const int64_t *__restrict__ labels, uint32_t *__restrict__ n_
         if (cls_count[c]) atomicAdd(dst + c, cls_count[c]);
 }
 
-// Decides which segments are binned and clears their bins.  grid (kBinChunks, S).
+// Decides which segments are binned and clears their bins.  grid S * kBinChunks.
 __global__ void __launch_bounds__(256) bin_setup_kernel(const BinArgs a) {
-    const int64_t seg = blockIdx.y;
+    const int64_t seg = blockIdx.x / kBinChunks;
+    const uint32_t chunk = blockIdx.x % kBinChunks;
     const BinMap map = make_bin_map(a, seg);
     const uint32_t nb = map.nb;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (chunk == 0 && threadIdx.x == 0) {
         a.seg_flags[seg] = nb ? kSegFlagBinned : 0u;
         a.map[seg] = map;
     }
-    const uint32_t end = min(nb, (blockIdx.x + 1u) * kBinChunk);
-    for (uint32_t b = blockIdx.x * kBinChunk + threadIdx.x; b < end; b += 256) {
+    const uint32_t end = min(nb, (chunk + 1u) * kBinChunk);
+    for (uint32_t b = chunk * kBinChunk + threadIdx.x; b < end; b += 256) {
         a.bg[seg * a.L + b] = 0u;
         a.fg[seg * a.L + b] = 0u;
     }
@@ -1187,11 +1189,12 @@ template <bool VEC> __global__ void __launch_bounds__(kSortThreads) bin_count_ke
     }
 }
 
-// Elements of a chunk of bins.  grid (kBinChunks, S).
+// Elements of a chunk of bins.  grid S * kBinChunks.
 __global__ void __launch_bounds__(256) bin_sum_kernel(const BinArgs a) {
     __shared__ uint32_t wb[8], wf[8];
-    const int64_t seg = blockIdx.y;
-    const uint32_t nb = load_bin_map(a, seg).nb, first = blockIdx.x * kBinChunk;
+    const int64_t seg = blockIdx.x / kBinChunks;
+    const uint32_t chunk = blockIdx.x % kBinChunks;
+    const uint32_t nb = load_bin_map(a, seg).nb, first = chunk * kBinChunk;
     if (first >= nb) return;
     uint32_t sb = 0, sf = 0;
 #pragma unroll 8
@@ -1213,30 +1216,31 @@ __global__ void __launch_bounds__(256) bin_sum_kernel(const BinArgs a) {
             sb += wb[w];
             sf += wf[w];
         }
-        a.chunk_sum[seg * kBinChunks + blockIdx.x] = make_uint2(sb, sf);
+        a.chunk_sum[seg * kBinChunks + chunk] = make_uint2(sb, sf);
     }
 }
 
-// Counts -> dJ, in place.  grid (kBinChunks, S); a warp takes 1024 consecutive bins in 32 rounds.
+// Counts -> dJ, in place.  grid S * kBinChunks; a warp takes 1024 consecutive bins in 32 rounds.
 __global__ void __launch_bounds__(256) bin_step_kernel(const BinArgs a) {
     __shared__ uint32_t wb[8], wf[8];
-    const int64_t seg = blockIdx.y;
+    const int64_t seg = blockIdx.x / kBinChunks;
+    const uint32_t chunk = blockIdx.x % kBinChunks;
     const BinMap map = load_bin_map(a, seg);
-    const uint32_t nb = map.nb, first = blockIdx.x * kBinChunk;
+    const uint32_t nb = map.nb, first = chunk * kBinChunk;
     if (first >= nb) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t w0 = first + uint32_t(warp) * (kBinChunk / 8);
     uint32_t *bg = a.bg + seg * a.L, *fg = a.fg + seg * a.L;
     // what lies in front of this chunk (at most kBinChunks - 1 = 31 chunks: one lane each)
     uint2 before = make_uint2(0u, 0u);
-    if (lane < int(blockIdx.x)) before = a.chunk_sum[seg * kBinChunks + lane];
+    if (lane < int(chunk)) before = a.chunk_sum[seg * kBinChunks + lane];
     uint32_t run_b = __reduce_add_sync(0xffffffffu, before.x), run_f = __reduce_add_sync(0xffffffffu, before.y);
     // few elements in coarse bins: sorted on all 30 bits instead.  (Every block takes this decision for itself; the first
     // one also tells the kernels that follow.)
     uint2 all = make_uint2(0u, 0u);
     if (uint32_t(lane) * kBinChunk < nb) all = a.chunk_sum[seg * kBinChunks + lane];
     if (__reduce_add_sync(0xffffffffu, all.x + all.y) < kFastMinKept && map.shift > kBinFineShift) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) a.seg_flags[seg] = 0u;
+        if (chunk == 0 && threadIdx.x == 0) a.seg_flags[seg] = 0u;
         return;
     }
     uint32_t cb[32], cf[32], tb = 0, tf = 0;
@@ -1354,10 +1358,10 @@ prune_compact_kernel(const uint32_t *__restrict__ keys, const uint32_t *__restri
                      const uint32_t *__restrict__ direct, uint32_t *__restrict__ keys_out,
                      uint32_t *__restrict__ vals_out, float *__restrict__ jacc, int64_t L, int64_t T, int prune, int per) {
     __shared__ uint32_t wtot[kSortWarps];
-    const int64_t seg = blockIdx.y;
+    const int64_t runs = (T + per - 1) / per, seg = blockIdx.x / runs, first = (blockIdx.x % runs) * per;
     if (__ldg(direct + seg) & (kSegFlagDirect | kSegFlagBinned)) return;
     const uint32_t limit = prune_limit(maxfg, minkey, seg, prune);
-  for (int64_t tile = int64_t(blockIdx.x) * per; tile < T && tile < (int64_t(blockIdx.x) + 1) * per; ++tile) {
+  for (int64_t tile = first; tile < T && tile < first + per; ++tile) {
     const int64_t t0 = tile * kSortTile;
     const int n = int(L - t0 < kSortTile ? L - t0 : kSortTile);
     const int64_t sbase = seg * L;
@@ -2043,7 +2047,7 @@ extern "C" int b200_lovasz_forward(const void *logits, const int64_t *labels, fl
         if ((rc = launch_status("lovasz class count launch")) != B200_OK) return rc;
         const BinArgs ba{w.keysA, w.maxfg, w.minkey, w.n_fg, w.direct, w.valsA, w.valsB,
                          reinterpret_cast<BinMap *>(w.binmap), reinterpret_cast<uint2 *>(w.hist), jacc, w.partial, g.L, g.T, prune};
-        const dim3 chunks(kBinChunks, unsigned(g.S));
+        const unsigned chunks = unsigned(g.S * kBinChunks);     // (at most S * T: a binned segment has 32 tiles and more)
         const bool vec = g.L % 4 == 0 && aligned16(jacc);      // (the workspace's arrays start on 256 bytes)
         bin_setup_kernel<<<chunks, 256, 0, s>>>(ba);
         if ((rc = launch_status("lovasz bin setup launch")) != B200_OK) return rc;
@@ -2059,7 +2063,7 @@ extern "C" int b200_lovasz_forward(const void *logits, const int64_t *labels, fl
         if ((rc = launch_status("lovasz bin jaccard launch")) != B200_OK) return rc;
     }
     const int per = g.S * g.T > 8192 ? 4 : 1;
-    const dim3 prune_grid(unsigned((g.T + per - 1) / per), unsigned(g.S));
+    const unsigned prune_grid = unsigned(g.S * ((g.T + per - 1) / per));
     prune_count_kernel<<<prune_grid, kSortThreads, 0, s>>>(w.keysA, w.maxfg, w.minkey, w.direct, w.kept, w.fgkept,
                                                          g.L, g.T, prune, per);
     if ((rc = launch_status("lovasz prune count launch")) != B200_OK) return rc;
