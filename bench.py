@@ -6,8 +6,8 @@
 A step is one forward + backward of a loss module over one synthetic batch
 (bench_workloads.py).  Rank 0 prints ONE JSON line.  Top-level fields describe the headline
 workload: the baseline file's third configuration (LargeMarginSoftmaxV3 fp32 [8,150,512,512]),
-the largest one it shards over GPUs.  `workloads` carries the same measurements for the other
-configurations and `table` (last key) repeats every workload in compact form.
+the largest one it shards over GPUs.  `table` (last key) has a row for every workload; their full
+records go to stderr, one JSON line each.
 
   value      logit elements / s, forward+backward, inputs resident in HBM, timed with CUDA
              events over K x R steps (R = `run.replays_per_step`, chosen so that the timed
@@ -19,13 +19,13 @@ configurations and `table` (last key) repeats every workload in compact form.
              (rotating input sets, preallocated outputs); peak from MEASURED_PEAKS.json
              (hbm_gbs) or the 6650 GB/s fallback; traffic from profiles/dram_traffic.json
   cpu_baseline  the CPU port (oracle/) on the host cores, bounded sample, N=1 only
-  reference_v3  (per workload, N=1 only) the reference project's own V3 CUDA extensions, built
+  reference_v3  (N=1 only) the reference project's own V3 CUDA extensions, built
              unmodified for sm_100a, timed by baseline/reference_v3.py in a process of its own
 
 Multi-GPU (torchrun, one rank per GPU): STRONG scaling.  The configuration's one global batch is
 split over the ranks along the batch axis (rank r holds N/G items), the modules add their
 [sum, count] pairs over the ranks, `value` = global elements / slowest rank's time.  The focal
-configuration (one 64 MB tensor) is additionally kept as a weak-scaling entry under `workloads`.
+configuration (one 64 MB tensor) is additionally kept as a weak-scaling row of `table`.
 
 `--impl reference` times the CPU port alone and prints the same line shape.
 L2 hygiene: every workload rotates 3 distinct input sets; where one set with its gradient is
@@ -670,6 +670,38 @@ def measure_workload(wl, args, device, world, rank, with_cpu, with_e2e, with_ent
     return res
 
 
+def result_line(results, headline, wl, wl_full, args, world, numa):
+    """The one line of rank 0: the headline workload's record and a row of `table` for every workload."""
+    h = results[headline]
+    table = {}
+    for k, v in results.items():
+        if "error" in v:
+            table[k] = "error"
+            continue
+        ref = v.get("reference_v3") or {}
+        e2e = v.get("e2e") or {}
+        table[k] = [round(v["ms_per_step"], 4), round(v["step_frac"], 3), v["scaling"],
+                    round(ref["ms_per_step"], 4) if "ms_per_step" in ref else None,
+                    round(e2e["ms_per_step"], 4) if "ms_per_step" in e2e else None]
+    return {
+        "metric": "logit elements/s forward+backward", "value": h["value"], "unit": "logit elements/s",
+        "n_gpus": world, "steps": args.steps, "warmup": args.warmup, "ms_per_step": h["ms_per_step"],
+        "higher_is_better": True, "scaling": "strong", "vs_baseline": None,
+        "dtype": "f16" if wl.dtype == torch.float16 else "f32", "data": "synthetic",
+        "config": base_config(wl_full),
+        "run": {"per_gpu_shape": list(wl.shape), "global_shape": list(wl_full.shape),
+                "l2": h["l2"], "cuda_graph": h["graph"], "replays_per_step": h["replays_per_step"],
+                "timed_region_ms": h["timed_region_ms"], "reduction_collective": reduction_collective(world),
+                "host_numa_binding": numa},
+        "roofline": h["roofline"], "cpu_baseline": h.get("cpu_baseline"), "e2e": h["e2e"],
+        "gpu_launches": h["launches_per_step"] * args.steps * h["replays_per_step"], "clocks": h["clocks"],
+        "reference_v3": h.get("reference_v3"),
+        "table_columns": ["ms_per_step", "fraction of HBM peak (algorithmic bytes of the step)", "scaling",
+                          "reference V3 CUDA ms_per_step (N=1)", "end-to-end ms_per_step"],
+        "table": table,
+    }
+
+
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--gpus", type=int, default=1)
@@ -744,36 +776,14 @@ def main():
     if rank == 0 and args.kernels_only:
         print(json.dumps({"kernels_only": True, "steps": args.steps, "warmup": args.warmup, "workloads": results}))
     elif rank == 0:
-        h = results[headline]
-        wl_full = BW.WORKLOADS[headline]
-        wl, sharded = shard_of[headline]
-        table = {}
+        wl, _ = shard_of[headline]
+        # the other workloads' records go to stderr, one a line: the result line stays short enough for a log's tail
         for k, v in results.items():
-            if "error" in v:
-                table[k] = "error"
-                continue
-            ref = v.get("reference_v3") or {}
-            table[k] = [round(v["ms_per_step"], 4), round(v["step_frac"], 3), v["scaling"],
-                        round(ref["ms_per_step"], 4) if "ms_per_step" in ref else None]
-        line = {
-            "metric": "logit elements/s forward+backward", "value": h["value"], "unit": "logit elements/s",
-            "n_gpus": world, "steps": args.steps, "warmup": args.warmup, "ms_per_step": h["ms_per_step"],
-            "higher_is_better": True, "scaling": "strong", "vs_baseline": None,
-            "dtype": "f16" if wl.dtype == torch.float16 else "f32", "data": "synthetic",
-            "config": base_config(wl_full if not args.items else wl),
-            "run": {"per_gpu_shape": list(wl.shape), "global_shape": list(wl_full.shape if not args.items else wl.shape),
-                    "l2": h["l2"], "cuda_graph": h["graph"], "replays_per_step": h["replays_per_step"],
-                    "timed_region_ms": h["timed_region_ms"], "reduction_collective": reduction_collective(world),
-                    "host_numa_binding": numa},
-            "roofline": h["roofline"], "cpu_baseline": h.get("cpu_baseline"), "e2e": h["e2e"],
-            "gpu_launches": h["launches_per_step"] * args.steps * h["replays_per_step"], "clocks": h["clocks"],
-            "reference_v3": h.get("reference_v3"),
-            "workloads": {k: v for k, v in results.items() if k != headline},
-            "table_columns": ["ms_per_step", "fraction of HBM peak (algorithmic bytes of the step)", "scaling",
-                              "reference V3 CUDA ms_per_step (N=1)"],
-            "table": table,
-        }
-        print(json.dumps(line))
+            if k != headline:
+                print(json.dumps({"workload": k, **{("description" if f == "workload" else f): u for f, u in v.items()}}),
+                      file=sys.stderr)
+        wl_full = wl if args.items else BW.WORKLOADS[headline]
+        print(json.dumps(result_line(results, headline, wl, wl_full, args, world, numa)))
     if world > 1:
         torch.distributed.barrier()
         torch.distributed.destroy_process_group()
