@@ -1007,8 +1007,9 @@ prune_scan_kernel(uint32_t *__restrict__ kept, const uint32_t *__restrict__ fgke
 // exactly its sorted dJ.  Counts are integers, so results do not depend on the order of the atomics.
 // Errors below 2^-31 share one last bin: their weight in the loss and in p(1-p) dJ is below that.
 //
-// Taken where n_pos >= kFastMinFg and the bins up to the pruning bound (8192 per octave of the error)
-// fit the segment's own part of the two value buffers, which the sort leaves unused then.
+// Taken where n_pos >= kFastMinFg, at least kFastMinKept elements count and the bins up to the pruning bound
+// (8192 per octave of the error) fit the segment's own part of the two value buffers, which the sort leaves unused
+// then: segments that the sort would put in exact order (see "Key bits") still go through it.
 // Measured, whole training step: 19 classes x 4 Mpixel images of 512 x 512 in one sort 561 -> 375 us, 152
 // segments of 1 Mpixel untrained 2222 -> 1310 us, trained 3717 -> 2310 us.  What bounds it: one reduction
 // and one look-up per element at ~190 G/s each (1.4 cycles per lane of an SM's load/store unit).
@@ -1042,7 +1043,6 @@ struct alignas(16) BinMap {
     __device__ __forceinline__ uint32_t bin(uint32_t key) const { return min(key >> shift, nb - 1u); }
 };
 constexpr uint32_t kBinFine = 65536u, kBinFinest = 131072u;
-constexpr int kBinFineShift = 8;              // 2^-16: resolves few elements as well as their sort would
 __device__ __forceinline__ BinMap make_bin_map(const BinArgs &a, int64_t seg) {
     BinMap m;
     const uint32_t last = prune_limit(a.maxfg, a.minkey, seg, a.prune) - 1u;       // largest (key >> 1) that counts
@@ -1053,7 +1053,7 @@ __device__ __forceinline__ BinMap make_bin_map(const BinArgs &a, int64_t seg) {
     if (m.capped) {
         m.nb = kBinCap;
     } else {
-        // (few foreground pixels: possibly few elements, which the sort would put in exact order)
+        // (fewer foreground pixels: dJ steps are larger)
         const uint32_t most = __ldg(a.n_fg + seg) < kFastMinKept ? kBinFinest : kBinFine;
         while (sh > 2 && (last >> (sh - 1)) < most && (last >> (sh - 1)) < a.L) m.nb = (last >> --sh) + 1u;
     }
@@ -1235,11 +1235,11 @@ __global__ void __launch_bounds__(256) bin_step_kernel(const BinArgs a) {
     uint2 before = make_uint2(0u, 0u);
     if (lane < int(chunk)) before = a.chunk_sum[seg * kBinChunks + lane];
     uint32_t run_b = __reduce_add_sync(0xffffffffu, before.x), run_f = __reduce_add_sync(0xffffffffu, before.y);
-    // few elements in coarse bins: sorted on all 30 bits instead.  (Every block takes this decision for itself; the first
-    // one also tells the kernels that follow.)
+    // few elements: sorted on all 30 bits, as any segment of so few (see "Key bits").  (Every block takes this decision
+    // for itself; the first one also tells the kernels that follow.)
     uint2 all = make_uint2(0u, 0u);
     if (uint32_t(lane) * kBinChunk < nb) all = a.chunk_sum[seg * kBinChunks + lane];
-    if (__reduce_add_sync(0xffffffffu, all.x + all.y) < kFastMinKept && map.shift > kBinFineShift) {
+    if (__reduce_add_sync(0xffffffffu, all.x + all.y) < kFastMinKept) {
         if (chunk == 0 && threadIdx.x == 0) a.seg_flags[seg] = 0u;
         return;
     }
