@@ -49,20 +49,19 @@ __device__ __forceinline__ float lanes_sum(float s, int tpr, unsigned mask) {
 // Large margin after the sums: the row's loss and the coefficients of its gradient
 // g_j = q_j (A + B d_j) + Cc with q_j = e^{d_j} / s', and of the target, -r.  `lbi` < 0: a label outside
 // the classes (undefined in the reference): every channel counts as off target.  `xd`: the value that
-// stood in for the target in the sums s and sde; its terms come back out here (s' >= 1 >= e^{xd - m'}, so
-// nothing cancels).  `sx`: the sum of the off-target logits.
+// stood in for the target in the sums; its terms come back out here (s' >= 1 >= e^{xd - m'}, so nothing cancels).
+// `sd`: the sum of the differences d_j = x_j - m' -- of the logits themselves it would carry an offset that they share.
+// The stand-in is the larger of two channels: a channel masked with the type's lowest value, added twice, would
+// overflow the sum.
 struct MarginRow {
     float loss, inv_s, sqx, r;
-    __device__ __forceinline__ void finish(float m, float s, float sde, float sx, float xl, float xd, int lbi, int C,
+    __device__ __forceinline__ void finish(float m, float s, float sde, float sd, float xl, float xd, int lbi,
                                            const LossConsts &k) {
-        float sd;
         if (lbi >= 0) {
             const float dc = xd - m, ec = ex2f(dc * kLog2e);
             s -= ec;
             sde -= dc * ec;
-            sd = sx - float(C - 1) * m;
-        } else {
-            sd = sx - float(C) * m;
+            sd -= dc;
         }
         inv_s = __fdividef(1.f, s);
         sqx = sde * inv_s;
@@ -74,6 +73,11 @@ struct MarginRow {
         loss = (mm + __logf(s_all)) - xl + k.half_lam * (sqx - k.a * sd);
     }
 };
+
+// The factor c of x c - m c in the exponent of 2: log2 e, or where m c would overflow one half -- logits that far
+// out are equal or 2^100 apart, so e^{x - m} is 1 or 0 either way.  (Rows of an odd length only, where such logits
+// have always been taken; the two registers cost 16-bit rows of even length 2 %.)
+__device__ __forceinline__ float exponent_scale(float m) { return fabsf(m) < 2.3e38f ? kLog2e : 0.5f; }
 
 // Two adjacent 16-bit elements in a word.
 template <typename T> struct Two;
@@ -280,7 +284,10 @@ rows_short_kernel(const SoftmaxParams prm) {
                 T dup{};
                 if (KIND == kLMargin && lbi >= 0) {
                     // the target's place holds another channel's logit during the sums
-                    dup = rp[(lbi == 0 && C > 1) ? 1 : 0];
+                    const int c0 = (lbi == 0 && C > 1) ? 1 : 0, c1 = C > 2 ? (lbi <= 1 ? 2 : 1) : c0;
+                    dup = rp[c0];
+                    const T other = rp[c1];
+                    if (to_f32(other) > to_f32(dup)) dup = other;
                     xd = to_f32(dup);
                 }
                 // every lane of the row has read x_lb before its owner writes there: the stand-in now or the
@@ -361,7 +368,7 @@ rows_short_kernel(const SoftmaxParams prm) {
                     float2 m2 = splat2(kNegInf), m3 = m2;        // (two chains each: latency)
 #pragma unroll
                     for (int i = 0; i < NP; ++i) {
-                        v[i] = psplat(kNegInf);
+                        v[i] = psplat(-INFINITY);
                         if constexpr (PAIRED) {
                             const uint32_t at = next(walk);
                             if (i < NU || i < np) v[i] = lds_pk<T>(at);
@@ -382,11 +389,11 @@ rows_short_kernel(const SoftmaxParams prm) {
                     }
                 }
                 m = lanes_max(m, TPR, row_mask);
-                const pk_t l2e = psplat(kLog2e), zero = psplat(0.f);
+                const pk_t zero = psplat(0.f);
                 float loss;
                 if constexpr (KIND == kLSR) {
-                    const float nm = -m * kLog2e;
-                    const pk_t nml = psplat(nm);
+                    const float c2 = PAIRED ? kLog2e : exponent_scale(m), nm = -m * c2;
+                    const pk_t l2e = psplat(c2), nml = psplat(nm);
                     pk_t ps[2] = {zero, zero}, px[2] = {zero, zero};
 #pragma unroll
                     for (int i = 0; i < NP; ++i) {
@@ -400,7 +407,7 @@ rows_short_kernel(const SoftmaxParams prm) {
                     float sum = s2.x + s2.y, sx = x2.x + x2.y;
                     if (odd) {
                         sx += vt;
-                        vt = ex2f(fmaf(vt, kLog2e, nm));
+                        vt = ex2f(fmaf(vt, c2, nm));
                         sum += vt;
                     }
                     for (int o = TPR >> 1; o > 0; o >>= 1) {
@@ -417,29 +424,28 @@ rows_short_kernel(const SoftmaxParams prm) {
 #pragma unroll
                         for (int i = 0; i < NP; ++i) put(walk, i, pfma(v[i], pa, pb));
                         if (odd) *last = from_f32<T>(fmaf(vt, a, b));
-                        if (owner) rp[lbi] = from_f32<T>(fmaf(ex2f(fmaf(xl, kLog2e, nm)), a, -kc.lb_pos * psc));
+                        if (owner) rp[lbi] = from_f32<T>(fmaf(ex2f(PAIRED ? fmaf(xl, kLog2e, nm) : (xl - m) * kLog2e), a, -kc.lb_pos * psc));
                     }
                 } else {
-                    const pk_t pnegm = psplat(-m);
-                    pk_t ps[2] = {zero, zero}, psde[2] = {zero, zero}, px[2] = {zero, zero};
+                    const pk_t l2e = psplat(kLog2e), pnegm = psplat(-m);
+                    pk_t ps[2] = {zero, zero}, psde[2] = {zero, zero}, psd[2] = {zero, zero};
 #pragma unroll
                     for (int i = 0; i < NP; ++i) {
                         const bool mine = i < NU || i < np;
-                        const pk_t x = mine ? x_of(i) : zero;
-                        px[i & 1] = padd(px[i & 1], x);
-                        const pk_t d = padd(x, pnegm);
-                        if constexpr (!kHold) v[i] = d;               // d = x - m' takes x's place
                         // (past the end: 0 by choice, the row's maximum may be the lowest value too)
+                        const pk_t d = mine ? padd(x_of(i), pnegm) : zero;
+                        psd[i & 1] = padd(psd[i & 1], d);
+                        if constexpr (!kHold) v[i] = d;               // d = x - m' takes x's place
                         const pk_t e = mine ? pex2(pmul(d, l2e)) : zero;
                         ps[i & 1] = padd(ps[i & 1], e);
                         psde[i & 1] = pfma(d, e, psde[i & 1]);
                     }
                     const float2 s2 = upk2(padd(ps[0], ps[1])), d2 = upk2(padd(psde[0], psde[1]));
-                    const float2 x2 = upk2(padd(px[0], px[1]));
-                    float sum = s2.x + s2.y, sde = d2.x + d2.y, sx = x2.x + x2.y;
+                    const float2 x2 = upk2(padd(psd[0], psd[1]));
+                    float sum = s2.x + s2.y, sde = d2.x + d2.y, sd = x2.x + x2.y;
                     if (odd) {
-                        sx += vt;
                         vt -= m;
+                        sd += vt;
                         const float e = ex2f(vt * kLog2e);
                         sum += e;
                         sde = fmaf(vt, e, sde);
@@ -447,10 +453,10 @@ rows_short_kernel(const SoftmaxParams prm) {
                     for (int o = TPR >> 1; o > 0; o >>= 1) {
                         sum += __shfl_xor_sync(row_mask, sum, o);
                         sde += __shfl_xor_sync(row_mask, sde, o);
-                        sx += __shfl_xor_sync(row_mask, sx, o);
+                        sd += __shfl_xor_sync(row_mask, sd, o);
                     }
                     MarginRow fin;
-                    fin.finish(m, sum, sde, lbi >= 0 ? sx - xd : sx, xl, xd, lbi, C, kc);
+                    fin.finish(m, sum, sde, sd, xl, xd, lbi, kc);
                     loss = fin.loss;
                     if constexpr (BWD) {
                         const float psc = prm.grad_mode == 2 ? gscale * to_f32(up) : gscale;
@@ -618,7 +624,10 @@ rows_vec_kernel(const SoftmaxParams prm) {
             const T *xs = static_cast<const T *>(prm.logits) + r * C;
             xl = to_f32(xs[lbi]);
         } else if (lbi >= 0) {
-            if constexpr (KIND == kLMargin) xd = __shfl_sync(0xffffffffu, VP::get(raw[0], lbi == 0 ? 1 : 0), 0);
+            if constexpr (KIND == kLMargin) {
+                const float x0 = VP::get(raw[0], lbi == 0 ? 1 : 0), x1 = VP::get(raw[0], lbi <= 1 ? 2 : 1);
+                xd = __shfl_sync(0xffffffffu, fmaxf(x0, x1), 0);
+            }
 #pragma unroll
             for (int i = 0; i < NV; ++i)
                 if (lane + 32 * i == lvec) {
@@ -662,11 +671,11 @@ rows_vec_kernel(const SoftmaxParams prm) {
 #pragma unroll
         for (int q = 1; q < kChains; ++q) m2[0] = max2(m2[0], m2[q]);
         const float m = lanes_max(fmaxf(m2[0].x, m2[0].y), 32, 0xffffffffu);
-        const pk_t l2e = psplat(kLog2e), zero = psplat(0.f);
+        const pk_t zero = psplat(0.f);
         float loss;
         if constexpr (KIND == kLSR) {
             const float nm = -m * kLog2e;
-            const pk_t nml = psplat(nm);
+            const pk_t l2e = psplat(kLog2e), nml = psplat(nm);
             pk_t ps[kChains], px[kChains];
 #pragma unroll
             for (int q = 0; q < kChains; ++q) ps[q] = px[q] = zero;
@@ -707,26 +716,26 @@ rows_vec_kernel(const SoftmaxParams prm) {
                         from_f32<T>(fmaf(ex2f(fmaf(xl, kLog2e, nm)), a, -kc.lb_pos * psc));
             }
         } else {
-            const pk_t pnegm = psplat(-m);
-            pk_t ps = zero, psde = zero, px = zero;
+            const pk_t l2e = psplat(kLog2e), pnegm = psplat(-m);
+            pk_t ps = zero, psde = zero, psd = zero;
 #pragma unroll
             for (int i = 0; i < NV; ++i)
                 if (i < cnt) {
 #pragma unroll
                     for (int p = 0; p < PV; ++p) {
                         pk_t &x = v[i * PV + p];
-                        px = padd(px, x);
                         x = padd(x, pnegm);                  // d = x - m' takes x's place
+                        psd = padd(psd, x);
                         const pk_t e = pex2(pmul(x, l2e));
                         ps = padd(ps, e);
                         psde = pfma(x, e, psde);
                     }
                 }
-            const float2 s2 = upk2(ps), d2 = upk2(psde), x2 = upk2(px);
+            const float2 s2 = upk2(ps), d2 = upk2(psde), x2 = upk2(psd);
             const float sum = lanes_sum(s2.x + s2.y, 32, 0xffffffffu), sde = lanes_sum(d2.x + d2.y, 32, 0xffffffffu);
-            const float sx = lanes_sum(x2.x + x2.y, 32, 0xffffffffu);
+            const float sd = lanes_sum(x2.x + x2.y, 32, 0xffffffffu);
             MarginRow fin;
-            fin.finish(m, sum, sde, lbi >= 0 ? sx - xd : sx, xl, xd, lbi, C, kc);
+            fin.finish(m, sum, sde, sd, xl, xd, lbi, kc);
             loss = fin.loss;
             if constexpr (BWD) {
                 const pk_t pa = psplat((fin.r + kc.half_lam * (1.f - fin.sqx)) * psc), pb = psplat(kc.half_lam * psc);

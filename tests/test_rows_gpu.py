@@ -108,3 +108,44 @@ def test_many_rows_against_64_bits(rows, kind, dtype):
             err = (grad.double() - ref).norm(dim=1) - 2 * TOL[dtype] * ref.norm(dim=1)
             assert float(err.max()) <= (1e-6 if reduction != "mean" else 1e-6 * scale), what
             assert not bool(grad[~valid].any()), what
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("c", [3, 5, 19, 20, 41, 150, 255, 256, 1000, 2047, 2048])
+def test_rows_with_channels_at_the_lowest_value(c, dtype):
+    """Channels masked with the type's lowest value (the one that stands in for the target in large margin's sums
+    among them): gradients as in 64 bits, and large margin's loss where its sum of differences is finite."""
+    import pytorch_loss as P
+    g = torch.Generator(device="cuda").manual_seed(c)
+    rows = 64
+    x = (torch.randn(rows, c, generator=g, device="cuda") * 2).to(dtype)
+    y = torch.randint(0, c, (rows,), generator=g, device="cuda")
+    low = torch.finfo(dtype).min
+    off = ~torch.nn.functional.one_hot(y, c).bool()
+    channel = torch.arange(c, device="cuda")[None, :]
+    for what, masked in (("one", (channel == (torch.arange(rows, device="cuda") % 4)[:, None])),
+                         ("several", (torch.rand(rows, c, generator=g, device="cuda") < 0.3) & (channel > 2)),
+                         ("all but the target", torch.ones(rows, c, dtype=torch.bool, device="cuda"))):
+        xm = x.masked_fill(masked & off, low)
+        for kind in ("lmargin", "lsr"):
+            if kind == "lmargin":
+                crit, oracle = P.LargeMarginSoftmaxV3(0.3, "none", -100), O.large_margin_softmax(xm, y, 0.3, -100, "none", torch.float64)
+            else:
+                crit, oracle = P.LabelSmoothSoftmaxCEV3(0.1, "none", -100), O.label_smooth_ce(xm, y, 0.1, -100, "none", torch.float64)
+            if kind == "lmargin" and what == "all but the target":
+                # (the oracle's own differences of 1e38 cancel badly: q = 1 / (c - 1), p = 0 off the target)
+                oracle = torch.zeros(rows, dtype=torch.float64, device="cuda"), torch.zeros_like(xm, dtype=torch.float64)
+            leaf = xm.clone().requires_grad_(True)
+            loss = crit(leaf, y)
+            grad, = torch.autograd.grad(loss, leaf, torch.ones_like(loss))
+            case = "%s c=%d %s, %s masked" % (kind, c, dtype, what)
+            if kind == "lmargin" and what != "several":      # (label smooth sums the logits themselves)
+                err = (loss.detach().double() - oracle[0]).abs() - TOL[dtype] * oracle[0].abs()
+                assert float(err.max()) <= 4e-6, case
+            assert float((grad.double() - oracle[1]).norm()) <= 2 * TOL[dtype] * float(oracle[1].norm()) + 1e-6, case
+    if c % 2:    # a row of nothing but lowest values: every channel is as likely as the others
+        leaf = torch.full((4, c), low, dtype=dtype, device="cuda").requires_grad_(True)
+        up = torch.ones(4, dtype=dtype, device="cuda")
+        grad, = torch.autograd.grad(P.LabelSmoothSoftmaxCEV3(0.1, "none", -100)(leaf, y[:4]), leaf, up)
+        want = O.label_smooth_ce(torch.zeros(4, c, device="cuda"), y[:4], 0.1, -100, "none", torch.float64)[1]
+        assert float((grad.double() - want).norm()) <= 2 * TOL[dtype] * float(want.norm())
