@@ -102,15 +102,12 @@ class LogTaylorSoftmaxV3(nn.Module):
 
 
 def _ce_step(logits, labels, n, ignore_index, mean):
-    """The 'mean' / 'sum' training step in one pass over the logits: (record, final gradient), or None
-    when the layout has none."""
+    """The 'mean' / 'sum' training step in one pass over the logits: (record, final gradient)."""
     nn_, c, m = _cabi.split_shape(logits, labels)
     logits, labels = logits.contiguous(), labels.contiguous()
     lib = _cabi.load_library()
     dev = logits.device
     grads = torch.empty_like(logits)
-    if not lib.b200_taylor_ce_step_path(_cabi.ptr(logits), _cabi.ptr(labels), _cabi.ptr(grads), nn_, c, m, _cabi.F32):
-        return None
     rec = _cabi.new_record(dev)
     ws = _cabi.reduce_workspace(dev)
     denom, flags = None, 0
@@ -163,16 +160,19 @@ class TaylorCrossEntropyLossV3(nn.Module):
         self.ignore_index = ignore_index
 
     def _fused(self, logits, labels):
+        """The one-kernel step takes this call: what b200_taylor_ce_step_path accepts, and nobody listens to the
+        activation or stands in for it."""
         act = self.taylor_softmax
         return (self.reduction in ('mean', 'sum') and type(act) is LogTaylorSoftmaxV3 and act.dim == 1 and
                 2 <= act.n <= 16 and act.n % 2 == 0 and
-                not (act._forward_hooks or act._forward_pre_hooks or act._backward_hooks or act._backward_pre_hooks) and
+                not (act._forward_hooks or act._forward_pre_hooks or act._backward_hooks or act._backward_pre_hooks or
+                     'forward' in act.__dict__ or nn.modules.module._has_any_global_hook()) and
                 logits.is_cuda and logits.requires_grad and torch.is_grad_enabled() and
                 (logits.dtype == torch.float32 or
                  (torch.is_autocast_enabled('cuda') and logits.dtype in (torch.float16, torch.bfloat16))) and
-                3 <= logits.dim() and logits.size(1) <= 64 and logits.numel() > 0 and
-                logits.numel() // (logits.size(0) * logits.size(1)) > 1 and
-                logits[0].numel() < 2 ** 31 and
+                3 <= logits.dim() and logits.size(1) <= 64 and
+                logits.size(0) * logits.size(1) < logits.numel() and      # (more than one pixel an image, no empty tensor)
+                logits.numel() // logits.size(0) < 2 ** 31 and
                 labels.device == logits.device and labels.dtype == torch.int64 and
                 labels.shape == logits.shape[:1] + logits.shape[2:])
 

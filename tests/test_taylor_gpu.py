@@ -114,3 +114,76 @@ def test_cross_entropy_step_against_64_bits(c, shape, order):
         assert_loss_close(loss, want.float(), atol=1e-6)
         assert_grad_close(first, ref.grad)
         assert_grad_close(again, ref.grad)
+
+
+def _taylor_64(x, y, n, reduction):
+    leaf = x.detach().double().contiguous().requires_grad_(True)
+    f = sum(leaf.pow(i) / math.factorial(i) for i in range(n + 1))
+    loss = torch.nn.functional.nll_loss((f / f.sum(1, keepdim=True)).log(), y, ignore_index=-1, reduction=reduction)
+    return loss.detach(), torch.autograd.grad(loss, leaf)[0]
+
+
+@pytest.mark.parametrize("form", ["channels_last", "slice", "expanded_labels", "offset", "half_autocast", "bfloat16_autocast"])
+def test_cross_entropy_step_takes_every_layout(form):
+    """Layouts, strides and types that the one-kernel step accepts, against 64 bits."""
+    import pytorch_loss as P
+    g = torch.Generator().manual_seed(23)
+    x = torch.randn(3, 7, 10, 12, generator=g).cuda()
+    y = torch.randint(-1, 7, (3, 10, 12), generator=g).cuda()
+    if form == "channels_last":
+        x = x.contiguous(memory_format=torch.channels_last)
+    elif form == "slice":
+        x, y = x[:, 1:6, ::2, 1:], (y.clamp(max=4))[:, ::2, 1:]
+    elif form == "expanded_labels":
+        y = y[:1].expand(3, 10, 12)
+    elif form == "offset":                                    # 4-byte aligned: one position a thread
+        x = torch.randn(3 * 7 * 120 + 1, generator=g).cuda()[1:].view(3, 7, 10, 12)
+    elif form.endswith("autocast"):
+        x = x.to(torch.float16 if form.startswith("half") else torch.bfloat16)
+    want, want_grad = _taylor_64(x, y, 4, "mean")
+    leaf = x.detach().requires_grad_(True)
+    crit = P.TaylorCrossEntropyLossV3(4, -1, "mean")
+    with torch.autocast("cuda", dtype=leaf.dtype if form.endswith("autocast") else torch.float16, enabled=form.endswith("autocast")):
+        assert crit._fused(leaf, y)
+        loss = crit(leaf, y)
+    grad, = torch.autograd.grad(loss, leaf)
+    assert loss.dtype == torch.float32 and grad.dtype == leaf.dtype and grad.shape == leaf.shape
+    assert_loss_close(loss, want)
+    if form.endswith("autocast"):                             # (the gradient is rounded to the logits' type)
+        assert float((grad.double() - want_grad).norm()) <= 4e-3 * float(want_grad.norm()) + 1e-7
+    else:
+        assert_grad_close(grad, want_grad)
+
+
+def test_cross_entropy_step_with_nothing_to_count():
+    import pytorch_loss as P
+    x = torch.randn(2, 5, 6, 6, generator=torch.Generator().manual_seed(1)).cuda().requires_grad_(True)
+    y = torch.full((2, 6, 6), -1, dtype=torch.int64).cuda()
+    for reduction in ("mean", "sum"):
+        loss = P.TaylorCrossEntropyLossV3(2, -1, reduction)(x, y)
+        grad, = torch.autograd.grad(loss, x)
+        assert torch.isnan(loss.detach()) if reduction == "mean" else float(loss.detach()) == 0.0
+        assert not bool(grad.any())
+
+
+@pytest.mark.parametrize("listener", ["global_hook", "instance_hook", "replaced_forward"])
+def test_cross_entropy_calls_an_activation_that_somebody_listens_to(listener):
+    import pytorch_loss as P
+    crit = P.TaylorCrossEntropyLossV3(2, -1, "mean")
+    act, calls = crit.taylor_softmax, []
+    handle = None
+    if listener == "global_hook":
+        handle = torch.nn.modules.module.register_module_forward_hook(lambda m, i, o: calls.append(m) if m is act else None)
+    elif listener == "instance_hook":
+        handle = act.register_forward_hook(lambda m, i, o: calls.append(m))
+    else:
+        original = act.forward
+        act.forward = lambda x: (calls.append(act), original(x))[1]
+    try:
+        g = torch.Generator().manual_seed(2)
+        x = torch.randn(2, 5, 6, 6, generator=g).cuda().requires_grad_(True)
+        crit(x, torch.randint(0, 5, (2, 6, 6), generator=g).cuda()).backward()
+    finally:
+        if handle is not None:
+            handle.remove()
+    assert calls == [act]
