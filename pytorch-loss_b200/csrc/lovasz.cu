@@ -900,35 +900,14 @@ sort_scan_kernel(uint32_t *__restrict__ hist, uint32_t *__restrict__ fghist,
 // sort tile, a scan per segment, and a stable compaction that also writes the dropped
 // elements' dJ (zero).  The sort then runs on the kept elements only (Lp per segment).
 
-// A block takes `per` consecutive tiles of one segment (a flat grid of S * ceil(T / per): there may be more segments
-// than gridDim.y can count): with many tiles, segments that are binned and have nothing to do here cost fewer
-// blocks (19 456 of them took 23 us to find out).
+// One tile to a block in both: several of them in a loop doubled the compaction's time (152 segments of 250 000,
+// 80 -> 169 us).  Where segments may be counted instead of sorted, bin_count_kernel counts for the others too: blocks
+// that find nothing to do cost 13 us for 19 456 of them.
 
 // kept[seg][tile] = number of elements of the tile with (key >> 1) < limit;
 // fgkept[seg][tile] = number of foreground elements of the tile.
-__global__ void __launch_bounds__(kSortThreads)
-prune_count_kernel(const uint32_t *__restrict__ keys, const uint32_t *__restrict__ maxfg,
-                   const uint32_t *__restrict__ minkey, const uint32_t *__restrict__ seg_flags,
-                   uint32_t *__restrict__ kept, uint32_t *__restrict__ fgkept, int64_t L, int64_t T, int prune,
-                   int per) {
+__device__ __forceinline__ void write_tile_counts(uint32_t c, uint32_t f, uint32_t *kept, uint32_t *fgkept, int64_t at) {
     __shared__ uint32_t wsum[kSortWarps], wfg[kSortWarps];
-    const int64_t runs = (T + per - 1) / per, seg = blockIdx.x / runs, first = (blockIdx.x % runs) * per;
-    if (__ldg(seg_flags + seg) & kSegFlagBinned) return;
-    const uint32_t limit = prune_limit(maxfg, minkey, seg, prune);
-  for (int64_t tile = first; tile < T && tile < first + per; ++tile) {
-    const int64_t t0 = tile * kSortTile;
-    const int n = int(L - t0 < kSortTile ? L - t0 : kSortTile);
-    const uint32_t *src = keys + seg * L + t0;
-    uint32_t c = 0, f = 0;
-#pragma unroll
-    for (int r = 0; r < kSortItems; ++r) {
-        const int idx = r * kSortThreads + threadIdx.x;
-        if (idx < n) {
-            const uint32_t k = __ldg(src + idx);
-            c += (k >> 1) < limit ? 1u : 0u;
-            f += key_is_fg(k) ? 1u : 0u;
-        }
-    }
     c = __reduce_add_sync(0xffffffffu, c);
     f = __reduce_add_sync(0xffffffffu, f);
     if ((threadIdx.x & 31) == 0) {
@@ -942,11 +921,34 @@ prune_count_kernel(const uint32_t *__restrict__ keys, const uint32_t *__restrict
             tot += wsum[w];
             fg += wfg[w];
         }
-        kept[seg * T + tile] = tot;
-        fgkept[seg * T + tile] = fg;
+        kept[at] = tot;
+        fgkept[at] = fg;
     }
-    __syncthreads();
-  }
+}
+__device__ __forceinline__ void prune_count_tile(const uint32_t *__restrict__ keys, uint32_t limit,
+                                                 uint32_t *__restrict__ kept, uint32_t *__restrict__ fgkept,
+                                                 int64_t L, int64_t T, int64_t seg, int64_t tile) {
+    const int64_t t0 = tile * kSortTile;
+    const int n = int(L - t0 < kSortTile ? L - t0 : kSortTile);
+    const uint32_t *src = keys + seg * L + t0;
+    uint32_t c = 0, f = 0;
+#pragma unroll
+    for (int r = 0; r < kSortItems; ++r) {
+        const int idx = r * kSortThreads + threadIdx.x;
+        if (idx < n) {
+            const uint32_t k = __ldg(src + idx);
+            c += (k >> 1) < limit ? 1u : 0u;
+            f += key_is_fg(k) ? 1u : 0u;
+        }
+    }
+    write_tile_counts(c, f, kept, fgkept, seg * T + tile);
+}
+__global__ void __launch_bounds__(kSortThreads)
+prune_count_kernel(const uint32_t *__restrict__ keys, const uint32_t *__restrict__ maxfg,
+                   const uint32_t *__restrict__ minkey, uint32_t *__restrict__ kept, uint32_t *__restrict__ fgkept,
+                   int64_t L, int64_t T, int prune) {
+    const int64_t seg = blockIdx.x / T, tile = blockIdx.x % T;
+    prune_count_tile(keys, prune_limit(maxfg, minkey, seg, prune), kept, fgkept, L, T, seg, tile);
 }
 
 // kept[seg][*] -> exclusive offsets, Lp[seg] = total.  One block of kBins threads per segment.
@@ -988,6 +990,57 @@ prune_scan_kernel(uint32_t *__restrict__ kept, const uint32_t *__restrict__ fgke
     }
 }
 
+// Kept (key, position) pairs of a tile, in order, to offsets[seg][tile]...; dJ = 0 everywhere
+// (the Jaccard kernel overwrites the kept ones).
+__global__ void __launch_bounds__(kSortThreads)
+prune_compact_kernel(const uint32_t *__restrict__ keys, const uint32_t *__restrict__ maxfg,
+                     const uint32_t *__restrict__ minkey, const uint32_t *__restrict__ offsets,
+                     const uint32_t *__restrict__ seg_flags, uint32_t *__restrict__ keys_out,
+                     uint32_t *__restrict__ vals_out, float *__restrict__ jacc, int64_t L, int64_t T, int prune) {
+    __shared__ uint32_t wtot[kSortWarps];
+    const int64_t seg = blockIdx.x / T, tile = blockIdx.x % T;
+    if (__ldg(seg_flags + seg) & (kSegFlagDirect | kSegFlagBinned)) return;
+    const uint32_t limit = prune_limit(maxfg, minkey, seg, prune);
+    const int64_t t0 = tile * kSortTile;
+    const int n = int(L - t0 < kSortTile ? L - t0 : kSortTile);
+    const int64_t sbase = seg * L;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int wbase = warp * (32 * kSortItems);
+    const uint32_t lt = lanemask_lt();
+    uint32_t key[kSortItems];
+    uint32_t keepbits = 0;                       // bit r: my element of round r stays
+    uint32_t wc = 0;
+#pragma unroll
+    for (int r = 0; r < kSortItems; ++r) {
+        const int idx = wbase + r * 32 + lane;
+        key[r] = idx < n ? __ldg(keys + sbase + t0 + idx) : kKeyIgnored;
+        if (idx < n) jacc[sbase + t0 + idx] = 0.f;
+    }
+#pragma unroll
+    for (int r = 0; r < kSortItems; ++r) {
+        const int idx = wbase + r * 32 + lane;
+        if (idx < n && (key[r] >> 1) < limit) keepbits |= 1u << r;
+    }
+#pragma unroll
+    for (int r = 0; r < kSortItems; ++r) wc += __popc(__ballot_sync(0xffffffffu, (keepbits >> r) & 1u));
+    if (lane == 0) wtot[warp] = wc;
+    __syncthreads();
+    uint32_t base = __ldg(offsets + seg * T + tile);
+    for (int w = 0; w < warp; ++w) base += wtot[w];
+    if (wc == 0) return;
+#pragma unroll
+    for (int r = 0; r < kSortItems; ++r) {
+        const bool keep = (keepbits >> r) & 1u;
+        const uint32_t m = __ballot_sync(0xffffffffu, keep);
+        if (keep) {
+            const uint32_t pos = base + __popc(m & lt);
+            keys_out[sbase + pos] = key[r];
+            vals_out[sbase + pos] = uint32_t(t0 + wbase + r * 32 + lane);
+        }
+        base += __popc(m);
+    }
+}
+
 // ------------------------------------------------------------------ binned segments
 //
 // A segment with many foreground pixels does not have to be sorted at all.  dJ of an element depends on
@@ -1010,12 +1063,14 @@ prune_scan_kernel(uint32_t *__restrict__ kept, const uint32_t *__restrict__ fgke
 // Taken where n_pos >= kFastMinFg, at least kFastMinKept elements count and the bins up to the pruning bound
 // (8192 per octave of the error) fit the segment's own part of the two value buffers, which the sort leaves unused
 // then: segments that the sort would put in exact order (see "Key bits") still go through it.
-// Measured, whole training step: 19 classes x 4 Mpixel images of 512 x 512 in one sort 561 -> 375 us, 152
-// segments of 1 Mpixel untrained 2222 -> 1310 us, trained 3717 -> 2310 us.  What bounds it: one reduction
-// and one look-up per element at ~190 G/s each (1.4 cycles per lane of an SM's load/store unit).
+// Measured, whole training step without the host, sorted -> counted: 19 classes of 4 images of 512 x 512 together,
+// trained, 557 -> 373 us; 152 segments of 1 Mpixel untrained 2190 -> 1335 us, trained 3690 -> 2350 us.  What bounds
+// it: one reduction and one look-up per element at ~190 G/s each (1.4 cycles per lane of an SM's load/store unit).
 constexpr uint32_t kBinCap = 31u * 8192u + 1u;
 constexpr int kBinChunk = 8192;                                    // bins per block of the scan kernels
 constexpr int kBinChunks = int((kBinCap + kBinChunk - 1) / kBinChunk);
+// From here on the bins of every map fit the segment.  Smaller segments, sorted / counted, whole step: 152 of 250 000
+// pixels 543 / 548 us untrained, 947 / 980 saturated; 304 of 65 536 330 / 384 and 675 / 715 us.
 constexpr int64_t kBinMinPixels = 1 << 18;
 
 struct BinMap;
@@ -1029,6 +1084,7 @@ struct BinArgs {
     double *partial;
     int64_t L, T;
     int prune;
+    uint32_t *kept, *fgkept;                 // of the segments that are sorted all the same
 };
 
 // How a segment's keys map to bins, from its pruning bound.  Where the errors span few octaves the bins are
@@ -1142,28 +1198,38 @@ template <bool VEC, typename F> __device__ __forceinline__ void for_tile_keys(co
     for (int r = 0; r < kQuads; r += 4) f(r * kSortThreads * 4, k + r);
 }
 
-// Counts the elements of one tile into its segment's bins.  grid S * T.
+// Counts the elements of one tile into its segment's bins, and for the prune scan: of a segment without bins, or of
+// one that turns out to have few elements (bin_step_kernel).  grid S * T.
 template <bool VEC> __global__ void __launch_bounds__(kSortThreads) bin_count_kernel(const BinArgs a) {
     const int64_t seg = blockIdx.x / a.T, tile = blockIdx.x % a.T;
     const BinMap map = load_bin_map(a, seg);
-    if (map.nb == 0u) return;
+    if (map.nb == 0u) {
+        prune_count_tile(a.keys, prune_limit(a.maxfg, a.minkey, seg, a.prune), a.kept, a.fgkept, a.L, a.T, seg, tile);
+        return;
+    }
     const int64_t t0 = tile * kSortTile;
     const int n = int(a.L - t0 < kSortTile ? a.L - t0 : kSortTile);
     uint32_t *bg = a.bg + seg * a.L, *fg = a.fg + seg * a.L;
+    uint32_t counted = 0;
     uint32_t last_bg = 0, last_fg = 0;            // the last bin is where a trained network's pixels pile up
-    auto add = [&](uint32_t k, uint32_t b, bool in) {      // (predicated, no branch)
-        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\t@p red.global.add.u32 [%0], 1;\n\t}" ::"l"(
+    auto add = [&](uint32_t k, uint32_t b, uint32_t count) {      // (predicated, no branch)
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\t@p red.global.add.u32 [%0], %1;\n\t}" ::"l"(
                          ((k & 1u) ? fg : bg) + b),
-                     "r"(in ? 1u : 0u)
+                     "r"(count)
                      : "memory");
     };
-    auto one = [&](uint32_t k) { add(k, k >> map.shift, map.has(k)); };
+    auto one = [&](uint32_t k) {
+        const uint32_t in = map.has(k) ? 1u : 0u;
+        counted += in;
+        add(k, k >> map.shift, in);
+    };
     auto one_capped = [&](uint32_t k) {
         const uint32_t b = k >> map.shift;
         const bool in = map.has(k), last = in && b >= kBinCap - 1u;
+        counted += in ? 1u : 0u;
         last_fg += (last && (k & 1u)) ? 1u : 0u;
         last_bg += (last && !(k & 1u)) ? 1u : 0u;
-        add(k, b, in && !last);
+        add(k, b, in && !last ? 1u : 0u);
     };
     auto all = [&](auto &&f) {
         for_tile_keys<VEC>(a.keys + seg * a.L + t0, n, [&](int, const uint4 *k) {
@@ -1178,15 +1244,19 @@ template <bool VEC> __global__ void __launch_bounds__(kSortThreads) bin_count_ke
     };
     if (!map.capped) {
         all(one);
-        return;
+    } else {
+        all(one_capped);
+        last_bg = __reduce_add_sync(0xffffffffu, last_bg);
+        last_fg = __reduce_add_sync(0xffffffffu, last_fg);
+        if ((threadIdx.x & 31) == 0) {
+            if (last_bg) atomicAdd(bg + (kBinCap - 1u), last_bg);
+            if (last_fg) atomicAdd(fg + (kBinCap - 1u), last_fg);
+        }
     }
-    all(one_capped);
-    last_bg = __reduce_add_sync(0xffffffffu, last_bg);
-    last_fg = __reduce_add_sync(0xffffffffu, last_fg);
-    if ((threadIdx.x & 31) == 0) {
-        if (last_bg) atomicAdd(bg + (kBinCap - 1u), last_bg);
-        if (last_fg) atomicAdd(fg + (kBinCap - 1u), last_fg);
-    }
+    // (without pruning a sort would take the ignored pixels too; few elements never make a segment `fast`, whatever
+    // their foreground)
+    write_tile_counts(counted, 0u, a.kept, a.fgkept, seg * a.T + tile);
+    if (map.bound == kKeyIgnored && threadIdx.x == 0) a.kept[seg * a.T + tile] = uint32_t(n);
 }
 
 // Elements of a chunk of bins.  grid S * kBinChunks.
@@ -1348,61 +1418,6 @@ template <bool VEC> __global__ void __launch_bounds__(kSortThreads) bin_jaccard_
         for (int w = 1; w < kSortWarps; ++w) d += sh[w];
         a.partial[seg * a.T + tile] = d;
     }
-}
-
-// Kept (key, position) pairs of a tile, in order, to offsets[seg][tile]...; dJ = 0 everywhere
-// (the Jaccard kernel overwrites the kept ones).
-__global__ void __launch_bounds__(kSortThreads)
-prune_compact_kernel(const uint32_t *__restrict__ keys, const uint32_t *__restrict__ maxfg,
-                     const uint32_t *__restrict__ minkey, const uint32_t *__restrict__ offsets,
-                     const uint32_t *__restrict__ direct, uint32_t *__restrict__ keys_out,
-                     uint32_t *__restrict__ vals_out, float *__restrict__ jacc, int64_t L, int64_t T, int prune, int per) {
-    __shared__ uint32_t wtot[kSortWarps];
-    const int64_t runs = (T + per - 1) / per, seg = blockIdx.x / runs, first = (blockIdx.x % runs) * per;
-    if (__ldg(direct + seg) & (kSegFlagDirect | kSegFlagBinned)) return;
-    const uint32_t limit = prune_limit(maxfg, minkey, seg, prune);
-  for (int64_t tile = first; tile < T && tile < first + per; ++tile) {
-    const int64_t t0 = tile * kSortTile;
-    const int n = int(L - t0 < kSortTile ? L - t0 : kSortTile);
-    const int64_t sbase = seg * L;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int wbase = warp * (32 * kSortItems);
-    const uint32_t lt = lanemask_lt();
-    uint32_t key[kSortItems];
-    uint32_t keepbits = 0;                       // bit r: my element of round r stays
-    uint32_t wc = 0;
-#pragma unroll
-    for (int r = 0; r < kSortItems; ++r) {
-        const int idx = wbase + r * 32 + lane;
-        key[r] = idx < n ? __ldg(keys + sbase + t0 + idx) : kKeyIgnored;
-        if (idx < n) jacc[sbase + t0 + idx] = 0.f;
-    }
-#pragma unroll
-    for (int r = 0; r < kSortItems; ++r) {
-        const int idx = wbase + r * 32 + lane;
-        if (idx < n && (key[r] >> 1) < limit) keepbits |= 1u << r;
-    }
-#pragma unroll
-    for (int r = 0; r < kSortItems; ++r) wc += __popc(__ballot_sync(0xffffffffu, (keepbits >> r) & 1u));
-    if (lane == 0) wtot[warp] = wc;
-    __syncthreads();
-    uint32_t base = __ldg(offsets + seg * T + tile);
-    for (int w = 0; w < warp; ++w) base += wtot[w];
-    if (wc != 0) {
-#pragma unroll
-        for (int r = 0; r < kSortItems; ++r) {
-            const bool keep = (keepbits >> r) & 1u;
-            const uint32_t m = __ballot_sync(0xffffffffu, keep);
-            if (keep) {
-                const uint32_t pos = base + __popc(m & lt);
-                keys_out[sbase + pos] = key[r];
-                vals_out[sbase + pos] = uint32_t(t0 + wbase + r * 32 + lane);
-            }
-            base += __popc(m);
-        }
-    }
-    __syncthreads();
-  }
 }
 
 // The sort tiles in use, listed segment by segment (entries: encode_tile).  The kept
@@ -2040,13 +2055,13 @@ extern "C" int b200_lovasz_forward(const void *logits, const int64_t *labels, fl
     const unsigned nblk_all = unsigned(g.S * g.T);
     const int prune = env_int("B200_LOVASZ_NO_PRUNE", 0) ? 0 : 1;
     const int allow_fast = env_int("B200_LOVASZ_EXACT", 0) ? 0 : 1;     // 0: every segment sorts on all 30 bits
-    // segments that need no sort (see "Binned segments"); the rest follows below
-    if (allow_fast && g.L >= kBinMinPixels) {
+    if (allow_fast && g.L >= kBinMinPixels) {             // some segments may need no sort (see "Binned segments")
         class_count_kernel<<<unsigned(g.N * ((g.M + kCountPixels - 1) / kCountPixels)), 256, size_t(g.C) * 4, s>>>(
             labels, w.n_fg, g.C, g.M, ignore_index, per_image);
         if ((rc = launch_status("lovasz class count launch")) != B200_OK) return rc;
         const BinArgs ba{w.keysA, w.maxfg, w.minkey, w.n_fg, w.direct, w.valsA, w.valsB,
-                         reinterpret_cast<BinMap *>(w.binmap), reinterpret_cast<uint2 *>(w.hist), jacc, w.partial, g.L, g.T, prune};
+                         reinterpret_cast<BinMap *>(w.binmap), reinterpret_cast<uint2 *>(w.hist), jacc, w.partial, g.L, g.T, prune,
+                         w.kept, w.fgkept};
         const unsigned chunks = unsigned(g.S * kBinChunks);     // (at most S * T: a binned segment has 32 tiles and more)
         const bool vec = g.L % 4 == 0 && aligned16(jacc);      // (the workspace's arrays start on 256 bytes)
         bin_setup_kernel<<<chunks, 256, 0, s>>>(ba);
@@ -2061,16 +2076,15 @@ extern "C" int b200_lovasz_forward(const void *logits, const int64_t *labels, fl
         if (vec) bin_jaccard_kernel<true><<<nblk_all, kSortThreads, 0, s>>>(ba);
         else bin_jaccard_kernel<false><<<nblk_all, kSortThreads, 0, s>>>(ba);
         if ((rc = launch_status("lovasz bin jaccard launch")) != B200_OK) return rc;
+    } else {
+        prune_count_kernel<<<nblk_all, kSortThreads, 0, s>>>(w.keysA, w.maxfg, w.minkey, w.kept, w.fgkept, g.L, g.T,
+                                                             prune);
+        if ((rc = launch_status("lovasz prune count launch")) != B200_OK) return rc;
     }
-    const int per = g.S * g.T > 8192 ? 4 : 1;
-    const unsigned prune_grid = unsigned(g.S * ((g.T + per - 1) / per));
-    prune_count_kernel<<<prune_grid, kSortThreads, 0, s>>>(w.keysA, w.maxfg, w.minkey, w.direct, w.kept, w.fgkept,
-                                                         g.L, g.T, prune, per);
-    if ((rc = launch_status("lovasz prune count launch")) != B200_OK) return rc;
     prune_scan_kernel<<<unsigned(g.S), kBins, 0, s>>>(w.kept, w.fgkept, w.Lp, w.direct, g.L, g.T, allow_fast);
     if ((rc = launch_status("lovasz prune scan launch")) != B200_OK) return rc;
-    prune_compact_kernel<<<prune_grid, kSortThreads, 0, s>>>(w.keysA, w.maxfg, w.minkey, w.kept, w.direct, w.keysB,
-                                                           w.valsB, jacc, g.L, g.T, prune, per);
+    prune_compact_kernel<<<nblk_all, kSortThreads, 0, s>>>(w.keysA, w.maxfg, w.minkey, w.kept, w.direct, w.keysB,
+                                                           w.valsB, jacc, g.L, g.T, prune);
     if ((rc = launch_status("lovasz prune compact launch")) != B200_OK) return rc;
 
     // The number of sorted elements is known on the device only: fixed grids (a multiple of the
@@ -2078,13 +2092,14 @@ extern "C" int b200_lovasz_forward(const void *logits, const int64_t *labels, fl
     tile_map_kernel<<<unsigned(g.S), 256, 0, s>>>(w.Lp, w.direct, w.tilemap, w.n_tiles, g.S);
     if ((rc = launch_status("lovasz tile map launch")) != B200_OK) return rc;
     auto grid_of = [&](int per_sm) {
-        // (measured on 8 x 19 x 1 Mpixel: a resident grid that loops costs 5.6 ms unpruned and 1.10 ms
-        // pruned, one block per possible tile 5.0 and 1.13 ms: more blocks than fit, capped -- where the
-        // binned segments leave nothing to sort, 32 times as many as fit took 16 us to say so, 8 times 4 us)
-        const int64_t want = int64_t(sm_count()) * per_sm * 8;
+        const int64_t want = int64_t(sm_count()) * per_sm;
         return unsigned(want < g.S * g.T ? want : g.S * g.T);
     };
-    const unsigned nblk_hist = grid_of(8), nblk = grid_of(2);
+    // More blocks than fit, capped.  The histograms are short: 8 times as many as fit (where counted segments leave
+    // nothing to sort, 32 times took 16 us to say so, 8 times 4 us).  The others run 3 % longer on a full list with 8
+    // times than with 32 (128 images of 19 x 65 536 pixels, whole step 5030 / 4855 us), which cost 11 us more where the
+    // list is empty.
+    const unsigned nblk_hist = grid_of(8 * 8), nblk = grid_of(2 * 32);
     unsigned *tickets = w.status + 16;           // zeroed with the status word; one per kernel
 
     // Buffer roles as a compacted segment that takes all three passes sees them: B -> A -> B,
