@@ -565,17 +565,26 @@ template <> struct VecPairs<__half> : VecPairs16<__half, __half2> {};
 template <> struct VecPairs<__nv_bfloat16> : VecPairs16<__nv_bfloat16, __nv_bfloat162> {};
 
 // NV: 16-byte vectors a lane can hold.
-template <typename T, int NV> constexpr int vec_blocks() {   // blocks per SM (registers)
+template <typename T, int KIND, bool BWD, int NV> constexpr int vec_blocks() {   // blocks per SM (registers)
+    // (16-bit large-margin step, 1000 classes: 152 bytes spilled with three, 26.6 us; 24.1 us with two)
+    if (KIND == kLMargin && BWD && sizeof(T) == 2 && NV == 4) return 2;
     return NV <= 4 ? 3 : 2;
 }
+// Vectors every lane holds for sure (launch_rows_vec picks the smallest NV of 8, 16, 32, 40, 48, 64 elements that
+// holds a row): no check on those.
+template <typename T, int NV> constexpr int vec_sure() {
+    constexpr int n = NV * (16 / int(sizeof(T)));
+    return (n == 64 ? 48 : n == 48 ? 40 : n == 40 ? 32 : n == 32 ? 16 : n == 16 ? 8 : 0) / (16 / int(sizeof(T)));
+}
 template <typename T, int KIND, bool BWD, int NV>
-__global__ void __launch_bounds__(kVecThreads, vec_blocks<T, NV>())
+__global__ void __launch_bounds__(kVecThreads, vec_blocks<T, KIND, BWD, NV>())
 rows_vec_kernel(const SoftmaxParams prm) {
     __shared__ double sh_red[64];
     using VP = VecPairs<T>;
     constexpr int VE = 16 / int(sizeof(T)), PV = VP::N;      // elements and pairs of a vector
-    // the next row's vectors in flight under this row's arithmetic, where the registers hold both
-    constexpr bool kAhead = NV * VE <= 40;
+    // the next row's vectors in flight under this row's arithmetic, where the registers hold both (float32 large margin
+    // at 40 elements spills: [16384, 1100] step 39.6 us with, 33.3 us without)
+    constexpr bool kAhead = NV * VE <= (KIND == kLMargin && sizeof(T) == 4 ? 32 : 40);
     // large margin replaces an element of the row below, which wants the vectors as loaded
     constexpr bool kRaw = kAhead || KIND == kLMargin;
     // accumulation chains: long rows wait on one chain's latency (float32 [32768, 2048] step 100 -> 95 us
@@ -584,6 +593,7 @@ rows_vec_kernel(const SoftmaxParams prm) {
     const int lane = threadIdx.x & 31;
     const int C = prm.k.C, nvec = C / VE;
     const int cnt = (nvec - lane + 31) >> 5;                 // my vectors: lane, lane + 32, ...
+    constexpr int NU = vec_sure<T, NV>();
     const int warps_b = int(blockDim.x) >> 5;
     const int64_t warps = int64_t(gridDim.x) * warps_b;
     const bool reduce = prm.out != nullptr;
@@ -601,7 +611,7 @@ rows_vec_kernel(const SoftmaxParams prm) {
         lb_next = __ldg(prm.labels + row);
 #pragma unroll
         for (int i = 0; i < NV; ++i)
-            if (i < cnt) {
+            if (i < NU || i < cnt) {
                 if constexpr (kRaw) raw[i] = __ldcs(xr + 32 * i);
                 else VP::unpack(__ldcs(xr + 32 * i), v + i * PV);
             }
@@ -642,7 +652,7 @@ rows_vec_kernel(const SoftmaxParams prm) {
         if constexpr (kRaw) {
 #pragma unroll
             for (int i = 0; i < NV; ++i)
-                if (i < cnt) VP::unpack(raw[i], v + i * PV);
+                if (i < NU || i < cnt) VP::unpack(raw[i], v + i * PV);
         }
         uint4 *grow = static_cast<uint4 *>(prm.grads) + r * nvec + lane;
         const int64_t row = r;
@@ -652,7 +662,7 @@ rows_vec_kernel(const SoftmaxParams prm) {
             if (BWD) {
 #pragma unroll
                 for (int i = 0; i < NV; ++i)
-                    if (i < cnt) __stcs(grow + 32 * i, make_uint4(0u, 0u, 0u, 0u));
+                    if (i < NU || i < cnt) __stcs(grow + 32 * i, make_uint4(0u, 0u, 0u, 0u));
             }
             continue;
         }
@@ -661,7 +671,7 @@ rows_vec_kernel(const SoftmaxParams prm) {
         for (int q = 0; q < kChains; ++q) m2[q] = splat2(kNegInf);
 #pragma unroll
         for (int i = 0; i < NV; ++i)
-            if (i < cnt) {
+            if (i < NU || i < cnt) {
 #pragma unroll
                 for (int p = 0; p < PV; ++p) {
                     float2 &mq = m2[(i * PV + p) % kChains];
@@ -681,7 +691,7 @@ rows_vec_kernel(const SoftmaxParams prm) {
             for (int q = 0; q < kChains; ++q) ps[q] = px[q] = zero;
 #pragma unroll
             for (int i = 0; i < NV; ++i)
-                if (i < cnt) {
+                if (i < NU || i < cnt) {
 #pragma unroll
                     for (int p = 0; p < PV; ++p) {
                         pk_t &x = v[i * PV + p];
@@ -704,7 +714,7 @@ rows_vec_kernel(const SoftmaxParams prm) {
                 const pk_t pa = psplat(a), pb = psplat(b);
 #pragma unroll
                 for (int i = 0; i < NV; ++i)
-                    if (i < cnt) {
+                    if (i < NU || i < cnt) {
                         pk_t g[PV];
 #pragma unroll
                         for (int p = 0; p < PV; ++p) g[p] = pfma(v[i * PV + p], pa, pb);
@@ -720,7 +730,7 @@ rows_vec_kernel(const SoftmaxParams prm) {
             pk_t ps = zero, psde = zero, psd = zero;
 #pragma unroll
             for (int i = 0; i < NV; ++i)
-                if (i < cnt) {
+                if (i < NU || i < cnt) {
 #pragma unroll
                     for (int p = 0; p < PV; ++p) {
                         pk_t &x = v[i * PV + p];
@@ -742,7 +752,7 @@ rows_vec_kernel(const SoftmaxParams prm) {
                 const pk_t pc = psplat(-kc.half_lam * kc.a * psc), pq = psplat(fin.inv_s);
 #pragma unroll
                 for (int i = 0; i < NV; ++i)
-                    if (i < cnt) {
+                    if (i < NU || i < cnt) {
                         pk_t g[PV];
 #pragma unroll
                         for (int p = 0; p < PV; ++p) {
@@ -779,12 +789,12 @@ template <typename T, int KIND, bool BWD> int launch_rows_vec(const SoftmaxParam
         launch_kernel(kern, dim3(unsigned(grid)), dim3(32 * warps), 0, stream, dep, prm);
     };
     constexpr int kSmall = sizeof(T) == 4 ? 8 : 4;           // 32 elements a lane
-    if (nv <= kSmall / 4) go(rows_vec_kernel<T, KIND, BWD, kSmall / 4>, vec_blocks<T, kSmall / 4>());
-    else if (nv <= kSmall / 2) go(rows_vec_kernel<T, KIND, BWD, kSmall / 2>, vec_blocks<T, kSmall / 2>());
-    else if (nv <= kSmall) go(rows_vec_kernel<T, KIND, BWD, kSmall>, vec_blocks<T, kSmall>());
-    else if (nv <= kSmall * 5 / 4) go(rows_vec_kernel<T, KIND, BWD, kSmall * 5 / 4>, vec_blocks<T, kSmall * 5 / 4>());
-    else if (nv <= kSmall * 3 / 2) go(rows_vec_kernel<T, KIND, BWD, kSmall * 3 / 2>, vec_blocks<T, kSmall * 3 / 2>());
-    else go(rows_vec_kernel<T, KIND, BWD, 2 * kSmall>, vec_blocks<T, 2 * kSmall>());
+    if (nv <= kSmall / 4) go(rows_vec_kernel<T, KIND, BWD, kSmall / 4>, vec_blocks<T, KIND, BWD, kSmall / 4>());
+    else if (nv <= kSmall / 2) go(rows_vec_kernel<T, KIND, BWD, kSmall / 2>, vec_blocks<T, KIND, BWD, kSmall / 2>());
+    else if (nv <= kSmall) go(rows_vec_kernel<T, KIND, BWD, kSmall>, vec_blocks<T, KIND, BWD, kSmall>());
+    else if (nv <= kSmall * 5 / 4) go(rows_vec_kernel<T, KIND, BWD, kSmall * 5 / 4>, vec_blocks<T, KIND, BWD, kSmall * 5 / 4>());
+    else if (nv <= kSmall * 3 / 2) go(rows_vec_kernel<T, KIND, BWD, kSmall * 3 / 2>, vec_blocks<T, KIND, BWD, kSmall * 3 / 2>());
+    else go(rows_vec_kernel<T, KIND, BWD, 2 * kSmall>, vec_blocks<T, KIND, BWD, 2 * kSmall>());
     return launch_status("softmax resident rows kernel launch");
 }
 
