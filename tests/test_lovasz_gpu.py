@@ -264,3 +264,56 @@ def test_segment_with_few_elements_to_sort_keeps_all_key_bits(monkeypatch):
     want, want_loss = gradient_of_class_0()
     assert int((want != 0).sum()) > 2 * 6000
     assert torch.equal(grad, want) and torch.equal(loss, want_loss)
+
+
+# equal logits: every element of a class falls into one bin (or two: foreground and background), whose counters a warp
+# adds to together
+@pytest.mark.parametrize("hw", [(512, 512), (513, 515)])
+def test_counted_segments_of_equal_logits(hw):
+    import pytorch_loss as P
+    g = torch.Generator().manual_seed(hw[0])
+    y = (torch.rand((1,) + hw, generator=g) < 0.3).long()
+    y[torch.rand(y.shape, generator=g) < 0.03] = 255
+    x = torch.zeros((1, 2) + hw).cuda().requires_grad_(True)
+    loss = P.LovaszSoftmaxV3("sum", 255, per_image=True)(x, y.cuda())
+    grad, = torch.autograd.grad(loss, x)
+    assert_loss_close(loss, torch.tensor(1.0), rtol=2e-6)          # every error is 1/2 and a class's dJ add up to 1
+    fg, bg = [], []                       # the mean dJ over all orders of foreground and background of each class
+    for c in (0, 1):
+        f, b = int((y == c).sum()), int((y == 1 - c).sum())
+        mean = float((1.0 / torch.arange(f, f + b + 1, dtype=torch.float64)).mean())
+        fg.append(mean)
+        bg.append(f / (f * (f + b)) + f / b * (1.0 / (f + b) - mean))
+    for c in (0, 1):
+        d = torch.tensor([-fg[0], bg[1]] if c == 0 else [bg[0], -fg[1]], dtype=torch.float64)    # d loss / d p
+        want = 0.5 * (d - 0.5 * d.sum())
+        got = grad.detach().cpu().double().permute(0, 2, 3, 1)[y == c]
+        # one float32 division each and a product
+        assert float((got - want).abs().max()) <= 1e-6 * float(want.abs().max())
+    assert not bool(grad.cpu().permute(0, 2, 3, 1)[y == 255].any())
+
+
+@pytest.mark.parametrize("hw", [(512, 512), (513, 515)])
+@pytest.mark.parametrize("kind", ["some", "saturated"])
+def test_counted_segments_of_partly_equal_logits(hw, kind, monkeypatch):
+    """Half of the pixels with equal logits, the others random or (the shared last bin) far apart: the loss of the
+    sorted form, which does not depend on the order of equal errors, and bit for bit the same again."""
+    import pytorch_loss as P
+    g = torch.Generator().manual_seed(7)
+    x = torch.randn((2, 5) + hw, generator=g) * (2 if kind == "some" else 40)
+    x[:, :, ::2] = 0
+    x[:, :, :40] = 0
+    y = torch.randint(0, 5, (2,) + hw, generator=g)
+    y[torch.rand(y.shape, generator=g) < 0.03] = 255
+    leaf = x.cuda().requires_grad_(True)
+
+    def step():
+        loss = P.LovaszSoftmaxV3("none", 255, per_image=True)(leaf, y.cuda())
+        return loss.detach(), torch.autograd.grad(loss.sum(), leaf)[0]
+
+    loss, grad = step()
+    again, grad_again = step()
+    assert torch.equal(loss, again) and torch.equal(grad, grad_again)
+    monkeypatch.setenv("B200_LOVASZ_EXACT", "1")
+    want, _ = step()
+    assert_loss_close(loss, want.cpu(), rtol=2e-6)
