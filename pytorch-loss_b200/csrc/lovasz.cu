@@ -925,9 +925,12 @@ __device__ __forceinline__ void write_tile_counts(uint32_t c, uint32_t f, uint32
         fgkept[at] = fg;
     }
 }
-__device__ __forceinline__ void prune_count_tile(const uint32_t *__restrict__ keys, uint32_t limit,
-                                                 uint32_t *__restrict__ kept, uint32_t *__restrict__ fgkept,
-                                                 int64_t L, int64_t T, int64_t seg, int64_t tile) {
+__global__ void __launch_bounds__(kSortThreads)
+prune_count_kernel(const uint32_t *__restrict__ keys, const uint32_t *__restrict__ maxfg,
+                   const uint32_t *__restrict__ minkey, uint32_t *__restrict__ kept, uint32_t *__restrict__ fgkept,
+                   int64_t L, int64_t T, int prune) {
+    const int64_t seg = blockIdx.x / T, tile = blockIdx.x % T;
+    const uint32_t limit = prune_limit(maxfg, minkey, seg, prune);
     const int64_t t0 = tile * kSortTile;
     const int n = int(L - t0 < kSortTile ? L - t0 : kSortTile);
     const uint32_t *src = keys + seg * L + t0;
@@ -942,13 +945,6 @@ __device__ __forceinline__ void prune_count_tile(const uint32_t *__restrict__ ke
         }
     }
     write_tile_counts(c, f, kept, fgkept, seg * T + tile);
-}
-__global__ void __launch_bounds__(kSortThreads)
-prune_count_kernel(const uint32_t *__restrict__ keys, const uint32_t *__restrict__ maxfg,
-                   const uint32_t *__restrict__ minkey, uint32_t *__restrict__ kept, uint32_t *__restrict__ fgkept,
-                   int64_t L, int64_t T, int prune) {
-    const int64_t seg = blockIdx.x / T, tile = blockIdx.x % T;
-    prune_count_tile(keys, prune_limit(maxfg, minkey, seg, prune), kept, fgkept, L, T, seg, tile);
 }
 
 // kept[seg][*] -> exclusive offsets, Lp[seg] = total.  One block of kBins threads per segment.
@@ -1158,18 +1154,18 @@ class_count_kernel(const int64_t *__restrict__ labels, uint32_t *__restrict__ n_
         if (cls_count[c]) atomicAdd(dst + c, cls_count[c]);
 }
 
-// Decides which segments are binned and clears their bins.  grid S * kBinChunks.
+constexpr unsigned kSetupBlocks = 8;
+// Decides which segments are binned and clears their bins.  grid S * kSetupBlocks.
 __global__ void __launch_bounds__(256) bin_setup_kernel(const BinArgs a) {
-    const int64_t seg = blockIdx.x / kBinChunks;
-    const uint32_t chunk = blockIdx.x % kBinChunks;
+    const int64_t seg = blockIdx.x / kSetupBlocks;
+    const uint32_t block = blockIdx.x % kSetupBlocks;
     const BinMap map = make_bin_map(a, seg);
     const uint32_t nb = map.nb;
-    if (chunk == 0 && threadIdx.x == 0) {
+    if (block == 0 && threadIdx.x == 0) {
         a.seg_flags[seg] = nb ? kSegFlagBinned : 0u;
         a.map[seg] = map;
     }
-    const uint32_t end = min(nb, (chunk + 1u) * kBinChunk);
-    for (uint32_t b = chunk * kBinChunk + threadIdx.x; b < end; b += 256) {
+    for (uint32_t b = block * 256u + threadIdx.x; b < nb; b += kSetupBlocks * 256u) {
         a.bg[seg * a.L + b] = 0u;
         a.fg[seg * a.L + b] = 0u;
     }
@@ -1203,12 +1199,23 @@ template <bool VEC, typename F> __device__ __forceinline__ void for_tile_keys(co
 template <bool VEC> __global__ void __launch_bounds__(kSortThreads) bin_count_kernel(const BinArgs a) {
     const int64_t seg = blockIdx.x / a.T, tile = blockIdx.x % a.T;
     const BinMap map = load_bin_map(a, seg);
-    if (map.nb == 0u) {
-        prune_count_tile(a.keys, prune_limit(a.maxfg, a.minkey, seg, a.prune), a.kept, a.fgkept, a.L, a.T, seg, tile);
-        return;
-    }
     const int64_t t0 = tile * kSortTile;
     const int n = int(a.L - t0 < kSortTile ? a.L - t0 : kSortTile);
+    if (map.nb == 0u) {                           // what prune_count_kernel counts
+        uint32_t c = 0, f = 0;
+        for_tile_keys<VEC>(a.keys + seg * a.L + t0, n, [&](int, const uint4 *k) {
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                c += (map.has(k[r].x) ? 1u : 0u) + (map.has(k[r].y) ? 1u : 0u) + (map.has(k[r].z) ? 1u : 0u) +
+                     (map.has(k[r].w) ? 1u : 0u);
+                f += (key_is_fg(k[r].x) ? 1u : 0u) + (key_is_fg(k[r].y) ? 1u : 0u) + (key_is_fg(k[r].z) ? 1u : 0u) +
+                     (key_is_fg(k[r].w) ? 1u : 0u);
+            }
+        });
+        write_tile_counts(c, f, a.kept, a.fgkept, seg * a.T + tile);
+        if (map.bound == kKeyIgnored && threadIdx.x == 0) a.kept[seg * a.T + tile] = uint32_t(n);
+        return;
+    }
     uint32_t *bg = a.bg + seg * a.L, *fg = a.fg + seg * a.L;
     uint32_t counted = 0;
     uint32_t last_bg = 0, last_fg = 0;            // the last bin is where a trained network's pixels pile up
@@ -2094,7 +2101,7 @@ extern "C" int b200_lovasz_forward(const void *logits, const int64_t *labels, fl
                          w.kept, w.fgkept};
         const unsigned chunks = unsigned(g.S * kBinChunks);     // (at most S * T: a binned segment has 32 tiles and more)
         const bool vec = g.L % 4 == 0 && aligned16(jacc);      // (the workspace's arrays start on 256 bytes)
-        bin_setup_kernel<<<chunks, 256, 0, s>>>(ba);
+        bin_setup_kernel<<<unsigned(g.S) * kSetupBlocks, 256, 0, s>>>(ba);
         if ((rc = launch_status("lovasz bin setup launch")) != B200_OK) return rc;
         if (vec) bin_count_kernel<true><<<nblk_all, kSortThreads, 0, s>>>(ba);
         else bin_count_kernel<false><<<nblk_all, kSortThreads, 0, s>>>(ba);
@@ -2125,11 +2132,12 @@ extern "C" int b200_lovasz_forward(const void *logits, const int64_t *labels, fl
         const int64_t want = int64_t(sm_count()) * per_sm;
         return unsigned(want < g.S * g.T ? want : g.S * g.T);
     };
-    // More blocks than fit, capped.  The histograms are short: 8 times as many as fit (where counted segments leave
-    // nothing to sort, 32 times took 16 us to say so, 8 times 4 us).  The others run 3 % longer on a full list with 8
-    // times than with 32 (128 images of 19 x 65 536 pixels, whole step 5030 / 4855 us), which cost 11 us more where the
-    // list is empty.
-    const unsigned nblk_hist = grid_of(8 * 8), nblk = grid_of(2 * 32);
+    // More blocks than fit, capped.  The histograms are short: 8 times as many as fit.  Scatter and rank run 3 % longer
+    // on a full list with 8 times than with 32 (whole step: 128 images of 19 x 65 536 pixels 5020 / 4850 us, 2 of
+    // 150 x 262 144 2480 / 2240 us), which cost 20 us more where the list is empty: 8 where classes of about equal size
+    // are counted, not sorted (8 images of 19 x 1 Mpixel 1310 / 1331 us).
+    const bool counted = allow_fast && g.L >= kBinMinPixels && g.L >= 2 * int64_t(kFastMinFg) * g.C;
+    const unsigned nblk_hist = grid_of(8 * 8), nblk = grid_of(2 * (counted ? 8 : 32));
     unsigned *tickets = w.status + 16;           // zeroed with the status word; one per kernel
 
     // Buffer roles as a compacted segment that takes all three passes sees them: B -> A -> B,
