@@ -201,6 +201,17 @@ inline void launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_
     cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
+// Lets `kernel` be launched with `bytes` of dynamic shared memory.  The limit belongs to the kernel, not to the launch:
+// it is always set to the same value, so that a thread that launches with less cannot lower it between another
+// thread's call and its launch.  (40 KB: static shared memory shares the default 48 KB.)
+constexpr size_t kMaxDynamicSmem = 220 * 1024;
+template <typename K> inline int set_smem(K kernel, size_t bytes) {
+    if (bytes > 40 * 1024 &&
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kMaxDynamicSmem)) != cudaSuccess)
+        return launch_status("cudaFuncSetAttribute(max dynamic shared memory)");
+    return B200_OK;
+}
+
 // ---- cross-GPU messages (see ExchangeSlot).  All three functions are called by ONE full warp.
 
 __device__ __forceinline__ unsigned exchange_flag(unsigned long long seq) {

@@ -1999,16 +1999,14 @@ int launch_tile(const TileArgs &a, cudaStream_t stream) {
         int64_t pgrid = int64_t(sm_count()) * ctas;
         if (pgrid > ptiles) pgrid = ptiles;
         auto kern = lovasz_pair_kernel<BWD>;
-        if (psmem > 40 * 1024 &&
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(psmem)) != cudaSuccess)
-            return launch_status("cudaFuncSetAttribute(lovasz pair)");
+        const int rc = set_smem(kern, psmem);
+        if (rc != B200_OK) return rc;
         kern<<<dim3(unsigned(pgrid)), kTileBlock, psmem, stream>>>(a, stages, m_logits, m_seg, m_grads);
         return launch_status(BWD ? "lovasz backward kernel launch" : "lovasz keys kernel launch");
     }
     auto launch = [&](auto kern) -> int {
-        if (smem > 48 * 1024 &&
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
-            return launch_status("cudaFuncSetAttribute(lovasz tile)");
+        const int rc = set_smem(kern, smem);
+        if (rc != B200_OK) return rc;
         kern<<<dim3(unsigned(grid)), kTileThreads, smem, stream>>>(a, m_logits, m_seg, m_grads);
         return launch_status(BWD ? "lovasz backward kernel launch" : "lovasz keys kernel launch");
     };

@@ -32,15 +32,6 @@ struct SoftmaxParams {
 
 inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-template <typename K> inline int set_smem(K kernel, size_t bytes) {
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
-    if (e != cudaSuccess) {
-        set_error("cudaFuncSetAttribute(%zu bytes of shared memory): %s", bytes, cudaGetErrorString(e));
-        return B200_ERR_LAUNCH;
-    }
-    return B200_OK;
-}
-
 // M == 1 layouts whose rows are kept in registers (rows_short.cuh; one translation unit per loss and
 // direction): forward (bwd = false; prm.losses and / or prm.out), backward (prm.out null) and the
 // fused training step (prm.out given).

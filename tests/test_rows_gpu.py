@@ -149,3 +149,30 @@ def test_rows_with_channels_at_the_lowest_value(c, dtype):
         grad, = torch.autograd.grad(P.LabelSmoothSoftmaxCEV3(0.1, "none", -100)(leaf, y[:4]), leaf, up)
         want = O.label_smooth_ce(torch.zeros(4, c, device="cuda"), y[:4], 0.1, -100, "none", torch.float64)[1]
         assert float((grad.double() - want).norm()) <= 2 * TOL[dtype] * float(want.norm())
+
+
+def test_threads_that_need_different_amounts_of_shared_memory():
+    """Two threads run one kernel at lengths whose stages take 131 and 82 KB: neither lowers the other's limit."""
+    import threading
+
+    import pytorch_loss as P
+    failures = []
+
+    def work(c):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                x = torch.randn(64, c, device="cuda").requires_grad_(True)
+                y = torch.randint(0, c, (64,), device="cuda")
+                crit = P.LabelSmoothSoftmaxCEV3(0.1, "sum", -100)
+                for _ in range(300):
+                    torch.autograd.grad(crit(x, y), x)
+                torch.cuda.current_stream().synchronize()
+        except Exception as exc:                              # noqa: BLE001  (reported by the main thread)
+            failures.append((c, repr(exc)))
+
+    threads = [threading.Thread(target=work, args=(c,)) for c in (2047, 1283)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures
