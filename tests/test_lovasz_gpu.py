@@ -205,8 +205,8 @@ def test_counted_segments_against_64_bits(shape, per_image, kind):
     loss = P.LovaszSoftmaxV3("sum", 255, per_image=per_image)(leaf, y.cuda())
     grad, = torch.autograd.grad(loss, leaf)
     assert_loss_close(loss, want, rtol=2e-6)                    # sums of fp32 terms; the order inside a bin cancels
-    # errors that agree to 2^-13 (counted) or in their float32 rounding (the 64-pixel class, sorted) change places:
-    # a step of dJ, at most 1/4096^2 of the one and 1/64^2 of the other, for few of the pixels
+    # the 64-pixel class, sorted, sets both bounds (test_counted_classes_alone holds the counted ones to theirs): errors
+    # that agree in their float32 rounding change places there, a step of dJ of at most 1/64^2
     assert float((grad.double().cpu() - want_grad).abs().max()) <= 1.0 / 64 ** 2
     # (swaps in the 64-pixel class, whose steps are the largest, alone make up 6e-5 of the norm in float32)
     assert float((grad.double().cpu() - want_grad).norm()) <= 2e-4 * float(want_grad.norm())
@@ -264,6 +264,35 @@ def test_segment_with_few_elements_to_sort_keeps_all_key_bits(monkeypatch):
     want, want_loss = gradient_of_class_0()
     assert int((want != 0).sum()) > 2 * 6000
     assert torch.equal(grad, want) and torch.equal(loss, want_loss)
+
+
+
+@pytest.mark.parametrize("shape,per_image", [((1, 3, 512, 512), True), ((2, 5, 513, 515), True), ((3, 4, 301, 293), False)])
+@pytest.mark.parametrize("kind", ["random", "trained"])
+def test_counted_classes_alone(shape, per_image, kind):
+    """Every class has tens of thousands of pixels and is counted.  The elements of a bin share a dJ: with b background
+    elements in it that is off by about b / 2U of itself, U >= the class's pixels.  Random errors leave some tens of
+    262 144 elements in each of 65 536 bins; confident mistakes share the bins next to 1, a few per cent of U, but
+    their p (1 - p) is 1e-4 and less.  So a pixel is off by some 1e-4 of the largest gradient, and few are."""
+    import pytorch_loss as P
+    from oracle import losses as O
+    n, c, h, w = shape
+    g = torch.Generator().manual_seed(h + 1)
+    x = torch.randn(shape, generator=g) * 1.4
+    y = torch.randint(0, c, (n, h // 16 + 1, w // 16 + 1), generator=g).repeat_interleave(16, 1).repeat_interleave(16, 2)
+    y = y[:, :h, :w].contiguous()
+    if kind == "trained":
+        other = torch.randint(0, c, (n, h, w), generator=g)
+        wrong = torch.rand((n, h, w), generator=g) < 0.04
+        x.scatter_add_(1, torch.where(wrong, other, y).unsqueeze(1), torch.rand((n, 1, h, w), generator=g) * 12 + 3)
+    y[torch.rand(y.shape, generator=g) < 0.03] = 255
+    want, want_grad = O.lovasz_softmax(x, y, 255, "sum", per_image=per_image, dtype=torch.float64)
+    leaf = x.cuda().requires_grad_(True)
+    loss = P.LovaszSoftmaxV3("sum", 255, per_image=per_image)(leaf, y.cuda())
+    grad, = torch.autograd.grad(loss, leaf)
+    assert_loss_close(loss, want, rtol=2e-6)
+    assert float((grad.double().cpu() - want_grad).abs().max()) <= 1e-3 * float(want_grad.abs().max())
+    assert float((grad.double().cpu() - want_grad).norm()) <= 5e-5 * float(want_grad.norm())
 
 
 # equal logits: every element of a class falls into one bin (or two: foreground and background), whose counters a warp
