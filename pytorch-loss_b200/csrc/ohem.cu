@@ -232,7 +232,9 @@ ohem_score_kernel(const T *__restrict__ logits, const int64_t *__restrict__ labe
 // The same for few classes (float32): a thread keeps all channels of VEC adjacent pixels (2: M even, 8-byte
 // aligned; 1: any M) in registers, every load in flight before the first is used, one exponential per
 // element.  Bound by HBM (the chunked walk above keeps 8 loads in flight and rescales its sums):
-// [8, 19, 769, 769] 167 -> 91 us.
+// [8, 19, 769, 769] 167 -> 91 us.  Two pixels up to 32 classes (64 values fill the registers), one up to 64; whole
+// relabelling of 4 images of 40 / 64 classes: 47 / 70 us here at 511 x 513, chunked 49 / 65 us at 512 x 512 (16-byte
+// loads) and 71 / 95 us at 514 x 515, an even number of pixels that is no multiple of 4.
 template <int CMAX, int VEC>
 __global__ void __launch_bounds__(kOhemThreads, CMAX * VEC <= 20 ? 5 : CMAX * VEC <= 40 ? 3 : 2)
 ohem_score_resident_kernel(const float *__restrict__ logits, const int64_t *__restrict__ labels, float *__restrict__ scores,

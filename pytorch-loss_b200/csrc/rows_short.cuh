@@ -13,7 +13,7 @@
 // Both were bound by instruction issue when a row stayed in shared memory and was walked three times
 // (35 thread instructions per bfloat16 element).  Measured, before -> after, kernel time:
 //   bfloat16 [32768, 1000] label-smooth step                  69.9 -> 30 us (4.4 TB/s)
-//   half [894916, 150] large margin, forward / backward       176 / 334 -> 95 / 166 us
+//   half [894916, 150] large margin, forward / backward       176 / 334 -> 95 / 160 us
 //
 // `prm.out` given: loss sum and count are reduced over the grid (the forward's record, or in backward
 // the fused training step).  Included by one translation unit per loss and direction.

@@ -555,8 +555,8 @@ int dispatch_taylor(TaylorParams &p, int dtype, int order, int use_log, const ch
 // is five passes (activation, nll forward, a zero fill and a scatter for the nll gradient, activation
 // backward: 20 bytes an element and more); this one moves 8.  A thread keeps all channels of VEC adjacent
 // pixels in registers (2: 8-byte accesses, up to 32 channels; 1: any pixel count and alignment, up to
-// 64), no shared memory before the final reduction.  HBM-bound: [16, 19, 512, 512] whole pass
-// 666 -> 180 us (the kernel 119).
+// 64), no shared memory before the final reduction.  HBM-bound: [16, 19, 512, 512] whole eager step
+// 667 -> 141 us (the kernel 119).
 template <int ORDER, int CMAX, int VEC>
 __global__ void __launch_bounds__(kTaylorThreads, CMAX * VEC <= 20 ? 4 : CMAX * VEC <= 42 ? 3 : 2)
 taylor_ce_step_kernel(const TaylorParams p, const int64_t *labels, int64_t ignore, const double *denom, void *workspace,
