@@ -346,3 +346,31 @@ def test_counted_segments_of_partly_equal_logits(hw, kind, monkeypatch):
     monkeypatch.setenv("B200_LOVASZ_EXACT", "1")
     want, _ = step()
     assert_loss_close(loss, want.cpu(), rtol=2e-6)
+
+
+@pytest.mark.parametrize("mask", [float("-inf"), torch.finfo(torch.float32).min, float("nan")])
+def test_counted_segments_with_masked_channels(mask, monkeypatch):
+    """Channels masked at some pixels, or NaN there: the counted form agrees with the sorted one (all key bits), which
+    the masks reach as errors of exactly 0 and 1; a NaN stays at its own pixels."""
+    import pytorch_loss as P
+    g = torch.Generator().manual_seed(11)
+    x = torch.randn((1, 4, 520, 512), generator=g)
+    y = torch.randint(0, 4, (1, 520, 512), generator=g)
+    hit = torch.rand(y.shape, generator=g) < 0.02
+    x[:, 3] = torch.where(hit, torch.tensor(mask), x[:, 3])
+    leaf = x.cuda().requires_grad_(True)
+
+    def step():
+        loss = P.LovaszSoftmaxV3("none", 255, per_image=True)(leaf, y.cuda())
+        return loss.detach().cpu(), torch.autograd.grad(loss.sum(), leaf)[0].cpu()
+
+    loss, grad = step()
+    monkeypatch.setenv("B200_LOVASZ_EXACT", "1")
+    want, want_grad = step()
+    assert_loss_close(loss, want, rtol=2e-6)
+    assert torch.equal(torch.isnan(grad), torch.isnan(want_grad))
+    if mask != mask:
+        assert not bool(torch.isnan(grad.permute(0, 2, 3, 1)[~hit]).any())
+    # (see test_counted_classes_alone: 65 000 pixels a class; the masked foreground pixels, errors of 1, share a bin)
+    diff = torch.nan_to_num(grad - want_grad).double()
+    assert float(diff.norm()) <= 1e-4 * float(torch.nan_to_num(want_grad).double().norm())
